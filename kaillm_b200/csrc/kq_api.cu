@@ -22,7 +22,7 @@ int cuda_fail(cudaError_t e, const char* what) {
 }
 
 Options& options() {
-  static Options o = {0, 3, 81, 2, 1, 0, 0, 1, 1, 0, 1, 1, 0, 1, 24, 1, 1, 1};
+  static Options o = {0, 3, 81, 2, 1, 0, 0, 1, 1, 0, 1, 1, 0, 1, 24, 1, 1, 1, 0};
   return o;
 }
 
@@ -140,6 +140,13 @@ static int mul_mat(const char* fn, bool mmq, const void* W, int type, int64_t n,
     if (rc) return rc;
   }
   if (gemm) return launch_gemm_tc(W, type, n, k, P, m, y, y_dtype, stride_y, mmq, st);
+  // Formats without a tensor-core GEMM: from mmq_min_m tokens on one integer GEMM instead of GEMV passes of 8 tokens.  A
+  // 64-token tile costs about the same however few tokens it holds, so small matrices, whose passes are cheap, change over
+  // later (Q5_K, GEMV passes / integer GEMM, us: 12288x4096 17 tokens 70 / 66; 6144x5120 32 tokens 74 / 83, 64 tokens
+  // 144 / 109; 1024x4096 64 tokens 44 / 87, 100 tokens 70 / 87, 333 tokens 230 / 98)
+  const int64_t mq_m = n >= 8192 ? 24 : n >= 4096 ? 48 : n >= 2048 ? 80 : 128;
+  if (impl == 0 && m >= (options().mmq_min_m ? options().mmq_min_m : mq_m) && mmq_supported(W, type))
+    return launch_mmq(W, type, n, k, P, m, y, y_dtype, stride_y, mmq, st);
   if (impl != 1 && gemv_mma_supported(W, type, n, k)) {
     // the streaming kernels take the rows whose total size is a multiple of 16 bytes (all of them for every even n);
     // up to 7 rows at the end of an odd-sized tensor go to the general kernel, so nothing is read past the tensor
@@ -455,9 +462,13 @@ static int moe_common(const char* fn, bool block, const void* W, int type, int64
   cudaStream_t st = (cudaStream_t)stream;
   Q8Ptrs P = q8_ptrs(scratch, p.L, n);
   Q8Ptrs Pq = P;   // only the row-major codes and scales are read
-  Pq.qsp = nullptr; Pq.xh = nullptr; Pq.s8h = nullptr; Pq.dT = nullptr; Pq.qsu = nullptr;
+  Pq.qsp = nullptr; Pq.xh = nullptr; Pq.s8h = nullptr; Pq.qsu = nullptr;
+  const bool gemm = block && options().moe_smem && ((uintptr_t)W % 16) == 0;
+  // the integer GEMM reads the code sums of Q2_K and Q5_0 from the tables the quantizer writes beside dT
+  if (!(gemm && (type == KQ_TYPE_Q2_K || type == KQ_TYPE_Q5_0))) Pq.dT = nullptr;
   rc = launch_quantize(x, x_dtype, tokens, k, stride_x, &Pq, nullptr, p.L.kpad, st);
   if (rc) return rc;
+  if (gemm) return launch_mmq_moe(W, type, experts, n, k, P, tokens, top_k, ids, nslots, expert_ids, num_post_padded, y, y_dtype, stride_y, st);
   return launch_moe(W, type, experts, n, k, P.ds, P.qs, p.L.kpad, tokens, top_k, ids, nslots, expert_ids, num_post_padded, block, y,
                     y_dtype, stride_y, st);
 }
@@ -535,6 +546,7 @@ int kq_set_option(const char* name, int value) {
   if (name && !strcmp(name, "tile_two_stage")) { options().tile_two_stage = value != 0; return KQ_OK; }
   if (name && !strcmp(name, "moe_smem")) { options().moe_smem = value != 0; return KQ_OK; }
   if (name && !strcmp(name, "row_stage_kb")) { options().row_stage_kb = value < 4 ? 4 : (value > 96 ? 96 : value); return KQ_OK; }
+  if (name && !strcmp(name, "mmq_min_m")) { options().mmq_min_m = value; return KQ_OK; }
   if (name && !strcmp(name, "umma")) { options().umma = value != 0; return KQ_OK; }
   if (name && !strcmp(name, "umma_min_m")) { options().umma_min_m = value; return KQ_OK; }
   if (name && !strcmp(name, "umma_box")) { options().umma_box = value != 0; return KQ_OK; }
@@ -557,6 +569,7 @@ int kq_get_option(const char* name, int* value) {
   if (name && value && !strcmp(name, "tile_two_stage")) { *value = options().tile_two_stage; return KQ_OK; }
   if (name && value && !strcmp(name, "moe_smem")) { *value = options().moe_smem; return KQ_OK; }
   if (name && value && !strcmp(name, "row_stage_kb")) { *value = options().row_stage_kb; return KQ_OK; }
+  if (name && value && !strcmp(name, "mmq_min_m")) { *value = options().mmq_min_m; return KQ_OK; }
   if (name && value && !strcmp(name, "umma")) { *value = options().umma; return KQ_OK; }
   if (name && value && !strcmp(name, "umma_min_m")) { *value = options().umma_min_m; return KQ_OK; }
   if (name && value && !strcmp(name, "umma_box")) { *value = options().umma_box; return KQ_OK; }

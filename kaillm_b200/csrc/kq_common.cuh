@@ -56,9 +56,11 @@ struct Options {
                        // or the format's wire bytes are staged through shared memory (where it is faster at every m)
   int row_stage_kb;    // Q4_K row-pair GEMV (1-2 tokens): target size of one ring stage (whole rows) in KB
   int tile_two_stage;  // 1: the shared-stage GEMV may run on two whole-row stages of >= 32 KB instead of splitting K
-  int moe_smem;        // 1: the MoE ops stage a block's / a pair's activations in shared memory (0: the one-warp-per-row kernel)
+  int moe_smem;        // 1: the MoE ops share activations through shared memory (block op: integer GEMM; 0: the one-warp-per-row kernel)
   int gemm_small_m;    // 1: calls of 17..gemm_min_m-1 tokens also go to the tcgen05 GEMM where it beats the 16-token
                        // GEMV passes (staged formats, enough 128-row tiles to fill the GPU)
+  int mmq_min_m;       // smallest token count at which the formats without a tcgen05 GEMM go to the integer GEMM
+                       // (0: by the number of rows)
 };
 Options& options();
 
@@ -273,6 +275,12 @@ bool gemv_kres_supported(const void* W, int type, int64_t n, int64_t k, int mtok
 int gemv_kres_splits(int type, int64_t n, int64_t k, int mtok);
 int launch_gemv_kres(const void* W, int type, int64_t n, int64_t k, const Q8Ptrs& P, int64_t m0, int mcount, void* y,
                      int y_dtype, int64_t stride_y, bool mmq, cudaStream_t st);
+int launch_mmq_moe(const void* W, int type, int64_t experts, int64_t n, int64_t k, const Q8Ptrs& P, int64_t tokens, int top_k,
+                   const int32_t* ids, int64_t nslots, const int32_t* expert_ids, const int32_t* num_post_padded, void* y, int y_dtype,
+                   int64_t stride_y, cudaStream_t st);
+bool mmq_supported(const void* W, int type);
+int launch_mmq(const void* W, int type, int64_t n, int64_t k, const Q8Ptrs& P, int64_t m, void* y, int y_dtype, int64_t stride_y,
+               bool mmq, cudaStream_t st);
 int launch_wait_arrival(const void* buf, size_t bytes, int elem_bytes, int* status, cudaStream_t st);
 int arrival_status(int* failed, int clear);
 int launch_p2p_allgather(const void* src, size_t bytes, int64_t rows, size_t dst_stride, void* const* peer_dst,
