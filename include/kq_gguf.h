@@ -283,6 +283,23 @@ int kq_moe_a8(const void* W, int type, int64_t experts, int64_t n, int64_t k, co
  * supported type; the reference's CUDA build answers 4), 0 for a type the library does not know. */
 int kq_moe_block_size(int type);
 
+/* The pieces of a whole feed-forward call (gate/up projection, SiLU-and-multiply, down projection, routing weights):
+ * kq_moe_project: kq_moe_a8_vec (expert_ids NULL: ids = topk_ids) or kq_moe_a8 (expert_ids given: ids = sorted ids); with
+ *   swiglu != 0 the activations are T(silu(x[:, 0:k])) * x[:, k:2k], formed and quantized in one launch.  Output rows of
+ *   per-pair calls whose expert id is invalid are written as zeros.
+ * kq_moe_align: what moe_align_block_size returns, in one launch; topk_ids int32 [total], num_sorted = num_blocks *
+ *   kq_moe_block_size >= total + experts * (block - 1); post[0] = padded total, post[1] = 1 if an id is invalid.  At most 8192
+ *   slots and 1024 experts (KQ_ELIMIT).
+ * kq_moe_combine: out[t, :] = sum over j of T(y[t * top_k + j, :] * T(weights[t, j])), y [tokens * top_k, n] dense. */
+int kq_moe_project(int swiglu, const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* x, int x_dtype,
+                   int64_t tokens, int64_t stride_x, const int32_t* ids, int64_t num_ids, const int32_t* expert_ids,
+                   const int32_t* num_tokens_post_padded, int top_k, void* y, int y_dtype, int64_t stride_y, void* scratch,
+                   size_t scratch_bytes, void* stream);
+int kq_moe_align(const int32_t* topk_ids, int64_t total, int64_t experts, int32_t* sorted_ids, int64_t num_sorted,
+                 int32_t* expert_ids, int64_t num_blocks, int32_t* post, void* stream);
+int kq_moe_combine(const void* y, int dtype, const void* weights, int w_dtype, int64_t tokens, int64_t n, int top_k, void* out,
+                   void* stream);
+
 /* Diagnostics: copies the device-side status word of a scratch buffer to the host (SYNCHRONISES with the
  * device; not for the serving path).  0 = every kernel that used the scratch finished normally; non-zero = a
  * bounded wait inside a kernel gave up and the kernel returned early (its outputs are then undefined).

@@ -443,7 +443,7 @@ int kq_mul_mat_prepared_gather(const void* W, int type, int64_t n_local, int64_t
 static int moe_common(const char* fn, bool block, const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* x,
                       int x_dtype, int64_t tokens, int64_t stride_x, const int32_t* ids, int64_t nslots, const int32_t* expert_ids,
                       const int32_t* num_post_padded, int top_k, void* y, int y_dtype, int64_t stride_y, void* scratch,
-                      size_t scratch_bytes, void* stream) {
+                      size_t scratch_bytes, void* stream, bool swiglu = false, int zero_bad = 0) {
   t_err[0] = 0;
   if (experts <= 0 || top_k <= 0 || nslots < 0) { set_error("%s: experts, top_k must be positive", fn); return KQ_EINVAL; }
   if (!ids || (block && (!expert_ids || !num_post_padded))) { set_error("%s: null index tensor", fn); return KQ_EINVAL; }
@@ -466,11 +466,17 @@ static int moe_common(const char* fn, bool block, const void* W, int type, int64
   const bool gemm = block && options().moe_smem && ((uintptr_t)W % 16) == 0;
   // the integer GEMM reads the code sums of Q2_K and Q5_0 from the tables the quantizer writes beside dT
   if (!(gemm && (type == KQ_TYPE_Q2_K || type == KQ_TYPE_Q5_0))) Pq.dT = nullptr;
-  rc = launch_quantize(x, x_dtype, tokens, k, stride_x, &Pq, nullptr, p.L.kpad, st);
+  if (swiglu) {   // this producer writes every table
+    if (stride_x < 2 * k) { set_error("%s: row stride %lld < 2 * k", fn, (long long)stride_x); return KQ_EINVAL; }
+    Pq.dT = P.dT;
+    rc = launch_prepare_swiglu(x, x_dtype, tokens, k, stride_x, Pq, st);
+  } else {
+    rc = launch_quantize(x, x_dtype, tokens, k, stride_x, &Pq, nullptr, p.L.kpad, st);
+  }
   if (rc) return rc;
   if (gemm) return launch_mmq_moe(W, type, experts, n, k, P, tokens, top_k, ids, nslots, expert_ids, num_post_padded, y, y_dtype, stride_y, st);
   return launch_moe(W, type, experts, n, k, P.ds, P.qs, p.L.kpad, tokens, top_k, ids, nslots, expert_ids, num_post_padded, block, y,
-                    y_dtype, stride_y, st);
+                    y_dtype, stride_y, st, zero_bad);
 }
 
 int kq_moe_a8_vec(const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* x, int x_dtype, int64_t tokens,
@@ -486,6 +492,34 @@ int kq_moe_a8(const void* W, int type, int64_t experts, int64_t n, int64_t k, co
               size_t scratch_bytes, void* stream) {
   return moe_common("kq_moe_a8", true, W, type, experts, n, k, x, x_dtype, tokens, stride_x, sorted_token_ids, num_sorted, expert_ids,
                     num_tokens_post_padded, top_k, y, y_dtype, stride_y, scratch, scratch_bytes, stream);
+}
+
+int kq_moe_project(int swiglu, const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* x, int x_dtype, int64_t tokens,
+                   int64_t stride_x, const int32_t* ids, int64_t num_ids, const int32_t* expert_ids, const int32_t* num_tokens_post_padded,
+                   int top_k, void* y, int y_dtype, int64_t stride_y, void* scratch, size_t scratch_bytes, void* stream) {
+  return moe_common("kq_moe_project", expert_ids != nullptr, W, type, experts, n, k, x, x_dtype, tokens, stride_x, ids,
+                    expert_ids ? num_ids : tokens * (int64_t)top_k, expert_ids, num_tokens_post_padded, top_k, y, y_dtype, stride_y, scratch,
+                    scratch_bytes, stream, swiglu != 0, 1);
+}
+
+int kq_moe_align(const int32_t* topk_ids, int64_t total, int64_t experts, int32_t* sorted_ids, int64_t num_sorted, int32_t* expert_ids,
+                 int64_t num_blocks, int32_t* post, void* stream) {
+  t_err[0] = 0;
+  if (!topk_ids || !sorted_ids || !expert_ids || !post) { set_error("kq_moe_align: null pointer"); return KQ_EINVAL; }
+  if (!moe_align_supported(total, experts)) { set_error("kq_moe_align: at most 8192 slots and 1024 experts"); return KQ_ELIMIT; }
+  if (num_blocks * KQ_MOE_BLOCK != num_sorted || num_sorted > 0x7fffffff || num_sorted < total + experts * (KQ_MOE_BLOCK - 1)) {
+    set_error("kq_moe_align: num_sorted must hold total + experts * %d slots in whole blocks", KQ_MOE_BLOCK - 1);
+    return KQ_EINVAL;
+  }
+  return launch_moe_align(topk_ids, total, experts, sorted_ids, num_sorted, expert_ids, num_blocks, post, (cudaStream_t)stream);
+}
+
+int kq_moe_combine(const void* y, int dtype, const void* weights, int w_dtype, int64_t tokens, int64_t n, int top_k, void* out, void* stream) {
+  t_err[0] = 0;
+  if (!y || !weights || !out) { set_error("kq_moe_combine: null pointer"); return KQ_EINVAL; }
+  if (!dtype_ok(dtype) || !dtype_ok(w_dtype)) { set_error("kq_moe_combine: unsupported dtype"); return KQ_EUNSUPPORTED; }
+  if (tokens <= 0 || n <= 0 || top_k <= 0 || tokens > 65535 || n > 0x7fffffff) { set_error("kq_moe_combine: size out of range"); return KQ_ELIMIT; }
+  return launch_moe_combine(y, dtype, weights, w_dtype, out, tokens, n, top_k, (cudaStream_t)stream);
 }
 
 int kq_wait_arrival(const void* buf, size_t bytes, int dtype, int* status, void* stream) {

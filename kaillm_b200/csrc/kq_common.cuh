@@ -239,7 +239,11 @@ int launch_prepare_swiglu(const void* gate_up, int x_dtype, int64_t m, int64_t k
 constexpr int KQ_MOE_BLOCK = 8;   // slots per block of expert-sorted tokens (what kq_moe_block_size reports)
 int launch_moe(const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* ds, const void* qs, int64_t kpad,
                int64_t tokens, int top_k, const int32_t* ids, int64_t nslots, const int32_t* expert_ids,
-               const int32_t* num_post_padded, bool block, void* y, int y_dtype, int64_t stride_y, cudaStream_t st);
+               const int32_t* num_post_padded, bool block, void* y, int y_dtype, int64_t stride_y, cudaStream_t st, int zero_bad = 0);
+bool moe_align_supported(int64_t total, int64_t experts);
+int launch_moe_align(const int32_t* ids, int64_t total, int64_t experts, int32_t* sorted, int64_t nsorted, int32_t* expert_ids, int64_t nblocks,
+                     int32_t* out, cudaStream_t st);
+int launch_moe_combine(const void* y, int dtype, const void* w, int w_dtype, void* out, int64_t tokens, int64_t n, int top_k, cudaStream_t st);
 int launch_gemv_dp4a(const void* W, int type, int64_t n, int64_t k, const void* ds, const void* qs,
                      int64_t kpad, int64_t m, void* y, int y_dtype, int64_t stride_y, bool mmq,
                      int32_t* dbg_dots, int32_t* dbg_sums, cudaStream_t st);

@@ -34,6 +34,7 @@ struct MoeParams {
   const int32_t* ids;                // vec: topk_ids [tokens * top_k]; block: sorted_token_ids
   const int32_t* expert_ids;         // block mode only
   const int32_t* num_post_padded;    // block mode only
+  int zero_bad;                      // vec: 1 = the output rows of pairs without a valid expert are written as zeros
   int64_t nslots;                    // tokens * top_k (vec) / entries of sorted_token_ids (block)
   void* y;
   int64_t stride_y;
@@ -72,7 +73,10 @@ __global__ void __launch_bounds__(128) moe_dp4a_kernel(const MoeParams p) {
     dst[0] = (int)z;
     tok[0] = (int)(z / p.top_k);
   }
-  if (expert < 0 || expert >= p.experts) return;
+  if (expert < 0 || expert >= p.experts) {
+    if (!BLOCK && p.zero_bad && lane == 0) reinterpret_cast<OutT*>(p.y)[(size_t)dst[0] * p.stride_y + row] = from_f32<OutT>(0.f);
+    return;
+  }
   const uint8_t* wrow = p.W + (size_t)expert * p.expert_stride + (size_t)row * p.rowbytes;
   const int nb8 = p.kpad >> 5;
   constexpr int NG = 32 / F::GROUP;
@@ -147,7 +151,11 @@ __global__ void __launch_bounds__(256) moe_vec_smem_kernel(const MoeParams p) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const int64_t z = blockIdx.y;                                              // the grid row is the (token, expert) pair
   const int expert = p.ids[z], tok = (int)(z / p.top_k);
-  if (expert < 0 || expert >= p.experts) return;
+  if (expert < 0 || expert >= p.experts) {
+    const int row = blockIdx.x * MOE_ROWS_PER_CTA + threadIdx.x;
+    if (p.zero_bad && threadIdx.x < MOE_ROWS_PER_CTA && row < p.n) reinterpret_cast<OutT*>(p.y)[(size_t)z * p.stride_y + row] = from_f32<OutT>(0.f);
+    return;
+  }
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.qs + (size_t)tok * p.kpad);
     for (int i = threadIdx.x; i < (p.kpad >> 4); i += blockDim.x) reinterpret_cast<uint4*>(sQ)[i] = __ldg(src + i);
@@ -254,17 +262,122 @@ int run_moe_out(const MoeParams& p, bool block, int y_dtype, cudaStream_t st) {
 
 }  // namespace
 
+// ---------------------------------------------------------------------------------------------- routing and combination
+// moe_align_block_size for a call of at most MOE_ALIGN_SLOTS slots and MOE_ALIGN_EXPERTS experts, in one CTA: slots sorted
+// by expert (in slot order inside an expert), every run padded to a multiple of `block` with `total`; expert id per block,
+// -1 past the padded total; out[0] = padded total, out[1] = 1 if some id is outside [0, experts).  A warp owns every 32nd
+// expert and finds its slots by ballots over the ids in shared memory.  Stands for 25 launches of torch ops.
+constexpr int MOE_ALIGN_SLOTS = 8192, MOE_ALIGN_EXPERTS = 1024;
+__global__ void __launch_bounds__(1024) moe_align_kernel(const int32_t* __restrict__ ids, int total, int experts, int block,
+                                                         int32_t* __restrict__ sorted, int nsorted, int32_t* __restrict__ expert_ids,
+                                                         int nblocks, int32_t* __restrict__ out) {
+  __shared__ int s_ids[MOE_ALIGN_SLOTS];
+  __shared__ int s_start[MOE_ALIGN_EXPERTS + 1];
+  __shared__ int s_bad;
+  const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
+  if (tid == 0) s_bad = 0;
+  __syncthreads();
+  bool bad = false;
+  for (int i = tid; i < total; i += 1024) {
+    const int e = ids[i];
+    s_ids[i] = e;
+    bad |= e < 0 || e >= experts;
+  }
+  if (bad) s_bad = 1;
+  for (int i = tid; i < nsorted; i += 1024) sorted[i] = total;
+  __syncthreads();
+  for (int e = warp; e < experts; e += 32) {
+    int count = 0;
+    for (int i = lane; i < ((total + 31) & ~31); i += 32) count += __popc(__ballot_sync(0xffffffffu, i < total && s_ids[i] == e));
+    if (lane == 0) s_start[e + 1] = (count + block - 1) / block * block;
+  }
+  __syncthreads();
+  if (warp == 0) {                       // running sum over the experts
+    int run = 0;
+    for (int e0 = 0; e0 < experts; e0 += 32) {
+      int v = e0 + lane < experts ? s_start[e0 + lane + 1] : 0;
+#pragma unroll
+      for (int d = 1; d < 32; d <<= 1) {
+        const int u = __shfl_up_sync(0xffffffffu, v, d);
+        if (lane >= d) v += u;
+      }
+      if (e0 + lane < experts) s_start[e0 + lane + 1] = run + v;
+      run += __shfl_sync(0xffffffffu, v, 31);
+    }
+    if (lane == 0) { s_start[0] = 0; out[0] = run; out[1] = s_bad; }
+  }
+  __syncthreads();
+  for (int e = warp; e < experts; e += 32) {
+    const int s0 = s_start[e], s1 = s_start[e + 1];
+    int at = s0;
+    for (int i = lane; i < ((total + 31) & ~31); i += 32) {
+      const bool mine = i < total && s_ids[i] == e;
+      const unsigned m = __ballot_sync(0xffffffffu, mine);
+      if (mine) sorted[at + __popc(m & ((1u << lane) - 1u))] = i;
+      at += __popc(m);
+    }
+    for (int b = s0 / block + lane; b < s1 / block; b += 32) expert_ids[b] = e;
+  }
+  for (int b = s_start[experts] / block + tid; b < nblocks; b += 1024) expert_ids[b] = -1;
+}
+
+// out[t, c] = sum over the token's experts of T(y[t * top_k + j, c] * w[t, j]): products rounded to T, fp32 sum, as
+// `(y.reshape(tokens, top_k, n) * w.to(T)).sum(1)`
+template <typename T, typename WT>
+__global__ void __launch_bounds__(256) moe_combine_kernel(const T* __restrict__ y, const WT* __restrict__ w, T* __restrict__ out, int n, int top_k) {
+  const int c = blockIdx.x * 256 + threadIdx.x;
+  const int64_t t = blockIdx.y;
+  if (c >= n) return;
+  float sum = 0.f;
+  for (int j = 0; j < top_k; ++j) {
+    const float wj = to_f32<T>(from_f32<T>(to_f32<WT>(w[t * top_k + j])));
+    sum += to_f32<T>(from_f32<T>(to_f32<T>(y[(t * top_k + j) * n + c]) * wj));
+  }
+  out[t * n + c] = from_f32<T>(sum);
+}
+
+template <typename T>
+static int run_combine(const void* y, const void* w, int w_dtype, void* out, int64_t tokens, int64_t n, int top_k, cudaStream_t st) {
+  const dim3 grid((unsigned)((n + 255) / 256), (unsigned)tokens);
+  switch (w_dtype) {
+    case KQ_F32: moe_combine_kernel<T, float><<<grid, 256, 0, st>>>((const T*)y, (const float*)w, (T*)out, (int)n, top_k); break;
+    case KQ_F16: moe_combine_kernel<T, __half><<<grid, 256, 0, st>>>((const T*)y, (const __half*)w, (T*)out, (int)n, top_k); break;
+    default: moe_combine_kernel<T, __nv_bfloat16><<<grid, 256, 0, st>>>((const T*)y, (const __nv_bfloat16*)w, (T*)out, (int)n, top_k); break;
+  }
+  options().launches += 1;
+  KQ_CUDA_TRY(cudaGetLastError());
+  return KQ_OK;
+}
+
+int launch_moe_combine(const void* y, int dtype, const void* w, int w_dtype, void* out, int64_t tokens, int64_t n, int top_k, cudaStream_t st) {
+  switch (dtype) {
+    case KQ_F32: return run_combine<float>(y, w, w_dtype, out, tokens, n, top_k, st);
+    case KQ_F16: return run_combine<__half>(y, w, w_dtype, out, tokens, n, top_k, st);
+    default: return run_combine<__nv_bfloat16>(y, w, w_dtype, out, tokens, n, top_k, st);
+  }
+}
+
+bool moe_align_supported(int64_t total, int64_t experts) { return total > 0 && total <= MOE_ALIGN_SLOTS && experts > 0 && experts <= MOE_ALIGN_EXPERTS; }
+
+int launch_moe_align(const int32_t* ids, int64_t total, int64_t experts, int32_t* sorted, int64_t nsorted, int32_t* expert_ids, int64_t nblocks,
+                     int32_t* out, cudaStream_t st) {
+  moe_align_kernel<<<1, 1024, 0, st>>>(ids, (int)total, (int)experts, KQ_MOE_BLOCK, sorted, (int)nsorted, expert_ids, (int)nblocks, out);
+  options().launches += 1;
+  KQ_CUDA_TRY(cudaGetLastError());
+  return KQ_OK;
+}
+
 // block = false: ids = topk_ids; block = true: ids = sorted_token_ids (MMQ arithmetic)
 int launch_moe(const void* W, int type, int64_t experts, int64_t n, int64_t k, const void* ds, const void* qs, int64_t kpad,
                int64_t tokens, int top_k, const int32_t* ids, int64_t nslots, const int32_t* expert_ids,
-               const int32_t* num_post_padded, bool block, void* y, int y_dtype, int64_t stride_y, cudaStream_t st) {
+               const int32_t* num_post_padded, bool block, void* y, int y_dtype, int64_t stride_y, cudaStream_t st, int zero_bad) {
   int blk, bytes;
   if (!type_geometry(type, &blk, &bytes)) { set_error("unsupported GGML type %d", type); return KQ_EUNSUPPORTED; }
   MoeParams p;
   p.W = (const uint8_t*)W; p.rowbytes = k / blk * bytes; p.expert_stride = p.rowbytes * n; p.n = (int)n; p.nsb = (int)(k / 32);
   p.experts = (int)experts; p.ds = (const __half2*)ds; p.qs = (const int8_t*)qs; p.kpad = (int)kpad; p.tokens = (int)tokens;
   p.top_k = top_k; p.ids = ids; p.expert_ids = expert_ids; p.num_post_padded = num_post_padded; p.nslots = nslots;
-  p.y = y; p.stride_y = stride_y;
+  p.y = y; p.stride_y = stride_y; p.zero_bad = zero_bad;
   const bool mmq = block;
 #define KQ_MOE_CASE(T) case T: return run_moe_out<T, false>(p, block, y_dtype, st)
 #define KQ_MOE_CASE2(T) case T: return mmq ? run_moe_out<T, true>(p, block, y_dtype, st) : run_moe_out<T, false>(p, block, y_dtype, st)

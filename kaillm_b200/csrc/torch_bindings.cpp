@@ -13,6 +13,7 @@
 
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
+#include <ATen/cuda/CUDAEvent.h>
 #include <c10/cuda/CUDAGuard.h>
 #include <torch/library.h>
 
@@ -146,6 +147,59 @@ at::Tensor ggml_moe_a8_vec(const at::Tensor& X, const at::Tensor& W, const at::T
   return moe_impl(false, X, W, topk_ids, nullptr, nullptr, type, row.expect_int(), top_k, tokens.expect_int());
 }
 
+// The whole SiLU feed-forward of linear.fused_moe_gguf: 5 launches (per-pair branch) or 6 (expert-sorted branch).
+// W1 [E, 2 * inter, row bytes], W2 [E, hidden_out, row bytes], topk_ids [tokens, top_k], topk_weights of as many entries.
+at::Tensor fused_moe_swiglu(const at::Tensor& X, const at::Tensor& W1, const at::Tensor& W2, const at::Tensor& topk_weights,
+                            const at::Tensor& topk_ids, int64_t type1, int64_t type2, bool block) {
+  const char* fn = "fused_moe_swiglu";
+  check_weight(W1, fn);
+  check_weight(W2, fn);
+  TORCH_CHECK(W1.dim() == 3 && W2.dim() == 3 && X.dim() == 2 && topk_ids.dim() == 2, fn, ": bad dimensions");
+  TORCH_CHECK(X.is_cuda() && X.stride(1) == 1, fn, ": X must be a CUDA tensor, contiguous along its last dimension");
+  for (const at::Tensor* t : {&W1, &W2, &topk_weights, &topk_ids}) TORCH_CHECK(t->is_cuda() && t->get_device() == X.get_device(), fn, ": all tensors must be on X's device");
+  const int64_t tokens = X.size(0), k1 = X.size(1), e = W1.size(0), n1 = W1.size(1), n2 = W2.size(1), top_k = topk_ids.size(1), pairs = tokens * top_k;
+  const int64_t k2 = n1 / 2;
+  int b1 = 0, s1 = 0, b2 = 0, s2 = 0;
+  TORCH_CHECK(kq_block_geometry((int)type1, &b1, &s1) == KQ_OK && kq_block_geometry((int)type2, &b2, &s2) == KQ_OK, fn, ": ", kq_last_error());
+  TORCH_CHECK(tokens > 0 && top_k > 0 && n1 % 2 == 0 && n1 > 0 && n2 > 0 && topk_ids.size(0) == tokens && topk_weights.numel() == pairs, fn, ": sizes do not match");
+  TORCH_CHECK(k1 % b1 == 0 && W1.size(2) == k1 / b1 * s1 && k2 % b2 == 0 && W2.size(2) == k2 / b2 * s2 && W2.size(0) == e, fn, ": weight sizes do not match");
+  const int xdt = kq_dtype_of(X.scalar_type(), fn), wdt = kq_dtype_of(topk_weights.scalar_type(), fn);
+  const c10::cuda::CUDAGuard guard(X.device());
+  auto stream = (void*)at::cuda::getCurrentCUDAStream(X.get_device()).stream();
+  const at::Tensor ids = topk_ids.to(at::kInt).contiguous();
+  const at::Tensor tw = topk_weights.contiguous();
+  const auto iopt = X.options().dtype(at::kInt);
+  at::Tensor sorted, eids, post, flag;
+  at::cuda::CUDAEvent copied;
+  if (block) {
+    const int64_t bs = kq_moe_block_size((int)type1), nb = (pairs + e * (bs - 1) + bs - 1) / bs;
+    sorted = at::empty({nb * bs}, iopt); eids = at::empty({nb}, iopt); post = at::empty({2}, iopt);
+    TORCH_CHECK(kq_moe_align(ids.data_ptr<int32_t>(), pairs, e, sorted.data_ptr<int32_t>(), nb * bs, eids.data_ptr<int32_t>(), nb,
+                             post.data_ptr<int32_t>(), stream) == KQ_OK, fn, ": ", kq_last_error());
+    // an expert id outside [0, E) is an error in this branch: the flag travels to the host while the kernels below run
+    flag = at::empty({2}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
+    flag.copy_(post, /*non_blocking=*/true);
+    copied.record(at::cuda::getCurrentCUDAStream(X.get_device()));
+  }
+  const size_t ws1 = kq_workspace_bytes((int)type1, tokens, n1, k1), ws2 = kq_workspace_bytes((int)type2, pairs, n2, k2);
+  at::Tensor scratch = at::empty({(int64_t)(ws1 > ws2 ? ws1 : ws2)}, W1.options());
+  at::Tensor h = at::empty({pairs, n1}, X.options()), y = at::empty({pairs, n2}, X.options()), out = at::empty({tokens, n2}, X.options());
+  const int32_t* idp = block ? sorted.data_ptr<int32_t>() : ids.data_ptr<int32_t>();
+  const int32_t* ep = block ? eids.data_ptr<int32_t>() : nullptr;
+  const int32_t* pp = block ? post.data_ptr<int32_t>() : nullptr;
+  const int64_t nid = block ? sorted.numel() : pairs;
+  TORCH_CHECK(kq_moe_project(0, W1.data_ptr(), (int)type1, e, n1, k1, X.data_ptr(), xdt, tokens, X.stride(0), idp, nid, ep, pp, (int)top_k,
+                             h.data_ptr(), xdt, n1, scratch.data_ptr(), scratch.numel(), stream) == KQ_OK, fn, ": ", kq_last_error());
+  TORCH_CHECK(kq_moe_project(1, W2.data_ptr(), (int)type2, e, n2, k2, h.data_ptr(), xdt, pairs, n1, idp, nid, ep, pp, 1, y.data_ptr(), xdt,
+                             n2, scratch.data_ptr(), scratch.numel(), stream) == KQ_OK, fn, ": ", kq_last_error());
+  TORCH_CHECK(kq_moe_combine(y.data_ptr(), xdt, tw.data_ptr(), wdt, tokens, n2, (int)top_k, out.data_ptr(), stream) == KQ_OK, fn, ": ", kq_last_error());
+  if (block) {
+    copied.synchronize();
+    TORCH_CHECK(flag.data_ptr<int32_t>()[1] == 0, fn, ": topk_ids holds an expert id outside [0, ", e, ")");
+  }
+  return out;
+}
+
 int64_t ggml_moe_get_block_size(int64_t type) { return kq_moe_block_size((int)type); }
 
 }  // namespace
@@ -158,6 +212,9 @@ TORCH_LIBRARY(_C_gguf, ops) {
       "ggml_moe_a8(Tensor X, Tensor W, Tensor sorted_token_ids, Tensor expert_ids, Tensor "
       "num_tokens_post_padded, int type, SymInt row, SymInt top_k, SymInt tokens) -> Tensor");
   ops.def("ggml_moe_a8_vec(Tensor X, Tensor W, Tensor topk_ids, int top_k, int type, SymInt row, SymInt tokens) -> Tensor");
+  ops.def(
+      "fused_moe_swiglu(Tensor X, Tensor W1, Tensor W2, Tensor topk_weights, Tensor topk_ids, int type1, int type2, bool block) "
+      "-> Tensor");
   ops.def("ggml_moe_get_block_size(int type) -> int");
 }
 
@@ -167,6 +224,7 @@ TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_mul_mat_a8", &ggml_mul_mat_a8);
   ops.impl("ggml_moe_a8", &ggml_moe_a8);
   ops.impl("ggml_moe_a8_vec", &ggml_moe_a8_vec);
+  ops.impl("fused_moe_swiglu", &fused_moe_swiglu);
 }
 
 TORCH_LIBRARY_IMPL(_C_gguf, CompositeExplicitAutograd, ops) {

@@ -17,6 +17,15 @@ IMATRIX_QUANT_TYPES = frozenset({20, 21, 23})    # IQ4_NL, IQ3_S, IQ4_XS
 MMVQ_QUANT_TYPES = frozenset({2, 3, 6, 7, 8, 10, 11, 12, 13, 14, 20, 21, 23})
 MMQ_QUANT_TYPES = frozenset({2, 3, 6, 7, 8, 10, 11, 12, 13, 14})
 DEQUANT_TYPES = MMVQ_QUANT_TYPES
+_FLOATS = (torch.float32, torch.float16, torch.bfloat16)
+
+
+def _plain(x: torch.Tensor) -> bool:
+    """An ordinary 2-D tensor nobody differentiates, traces or batches: only then may an op without derivative and tracing
+    rules stand in for a chain of torch ops."""
+    return (type(x) is torch.Tensor and x.is_cuda and x.dim() == 2 and not torch.compiler.is_compiling()
+            and not (x.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(x)
+            and torch.autograd.forward_ad.unpack_dual(x).tangent is None)
 
 
 def fused_mul_mat_gguf(x: torch.Tensor, qweight: torch.Tensor, qweight_type: int) -> torch.Tensor:
@@ -115,6 +124,23 @@ def moe_align_block_size(topk_ids: torch.Tensor, block_size: int, num_experts: i
     return sorted_ids, expert_ids, ends[-1:].to(torch.int32)
 
 
+def _moe_in_one_call(x, w1, w2, topk_weights, topk_ids, t1: int, t2: int, block: bool) -> bool:
+    """The calls `ops.fused_moe_swiglu` takes: plain dense tensors of matching sizes; the sorted branch up to the sizes of
+    the one-CTA sort."""
+    if not (_plain(x) and _plain(topk_weights) and _plain(topk_ids) and t1 in MMVQ_QUANT_TYPES and t2 in MMVQ_QUANT_TYPES
+            and w1.dim() == 3 and w2.dim() == 3):
+        return False
+    (tokens, hidden), (e, n, rb1), top_k = x.shape, w1.shape, topk_ids.shape[1]
+    (blk1, nb1), (blk2, nb2) = BLOCK[t1], BLOCK[t2]
+    return (0 < tokens <= 65535 and 0 < tokens * top_k <= (8192 if block else 65535) and not (block and e > 1024)
+            and x.stride(1) == 1 and w1.is_contiguous() and w2.is_contiguous() and w1.dtype == w2.dtype == torch.uint8
+            and x.dtype in _FLOATS and topk_weights.dtype in _FLOATS and topk_ids.dtype in (torch.int32, torch.int64)
+            and x.device == w1.device == w2.device == topk_weights.device == topk_ids.device
+            and topk_ids.shape[0] == tokens and topk_weights.numel() == tokens * top_k
+            and n > 0 and n % 2 == 0 and hidden % blk1 == 0 and n // 2 % blk2 == 0 and rb1 == hidden // blk1 * nb1
+            and w2.shape[0] == e and w2.shape[1] > 0 and w2.shape[2] == n // 2 // blk2 * nb2)
+
+
 def fused_moe_gguf(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
                    qweight_type: int, qweight_type2: int) -> torch.Tensor:
     """`_fused_moe_gguf` with the SiLU-and-multiply activation (quantization/fused_moe.py:34-133): gate/up projection of
@@ -124,13 +150,16 @@ def fused_moe_gguf(x: torch.Tensor, w1: torch.Tensor, w2: torch.Tensor, topk_wei
     e, n = w1.shape[0], w1.shape[1]
     top_k = topk_ids.shape[1]
 
+    block = qweight_type in MMQ_QUANT_TYPES and qweight_type2 in MMQ_QUANT_TYPES and num_tokens > 64
+    if _moe_in_one_call(x, w1, w2, topk_weights, topk_ids, qweight_type, qweight_type2, block):
+        return ops.fused_moe_swiglu(x, w1, w2, topk_weights, topk_ids, qweight_type, qweight_type2, block)
+
     def act(t):
         d = t.shape[-1] // 2
         return torch.nn.functional.silu(t[..., :d]) * t[..., d:]
 
-    if qweight_type in MMQ_QUANT_TYPES and qweight_type2 in MMQ_QUANT_TYPES and num_tokens > 64:
-        block = ops.ggml_moe_get_block_size(qweight_type)
-        s, ex, tot = moe_align_block_size(topk_ids, block, e)
+    if block:
+        s, ex, tot = moe_align_block_size(topk_ids, ops.ggml_moe_get_block_size(qweight_type), e)
         out = ops.ggml_moe_a8(x, w1, s, ex, tot, qweight_type, n, top_k, num_tokens)
         out = ops.ggml_moe_a8(act(out), w2, s, ex, tot, qweight_type2, w2.shape[1], 1, num_tokens * top_k)
     elif qweight_type in MMVQ_QUANT_TYPES and qweight_type2 in MMVQ_QUANT_TYPES:

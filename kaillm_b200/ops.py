@@ -63,3 +63,9 @@ def ggml_moe_a8_vec(X: torch.Tensor, W: torch.Tensor, topk_ids: torch.Tensor, to
 def ggml_moe_get_block_size(quant_type: int) -> int:
     """vllm_gguf_plugin/ops.py:281-284."""
     return torch.ops._C_gguf.ggml_moe_get_block_size(quant_type)
+
+
+def fused_moe_swiglu(X: torch.Tensor, W1: torch.Tensor, W2: torch.Tensor, topk_weights: torch.Tensor, topk_ids: torch.Tensor,
+                     quant_type: int, quant_type2: int, block: bool) -> torch.Tensor:
+    """The whole SiLU feed-forward of `linear.fused_moe_gguf` as one call (no gradient); `block`: expert-sorted branch."""
+    return torch.ops._C_gguf.fused_moe_swiglu(X, W1, W2, topk_weights, topk_ids, quant_type, quant_type2, block)
