@@ -248,6 +248,19 @@ int kq_wait_arrival(const void* buf, size_t bytes, int dtype, int* status, void*
  * clear != 0, zeroes it.  0 = no poll has run out since the last clear. */
 int kq_arrival_status(int* failed, int clear);
 
+/* y[m, n] = x[m, k] @ dequantize(W)^T without the dequantized matrix in memory - the ggml_dequantize + matmul pair the
+ * reference runs for the i-matrix formats above their mat-vec limits (quantization/linear.py:54-60).  The weights are
+ * rounded to x's type exactly as kq_dequantize does, products accumulate in fp32, y has x's type.  dtype: KQ_F16 or KQ_BF16.
+ * kq_dequant_mul_mat_supported returns 1 for what the kernel takes (IQ3_S, IQ4_NL, IQ4_XS; k a multiple of 256; W, x and
+ * every row of x 16-byte aligned).  No scratch; a bounded wait that ran out leaves a non-zero word that
+ * kq_dequant_mul_mat_status copies to *status (SYNCHRONISES; may be NULL) and, with clear != 0, zeroes. */
+int kq_dequant_mul_mat_supported(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m,
+                                 int64_t stride_x);
+int kq_dequant_mul_mat_preferred(int64_t n, int64_t m);   /* 1 where it is faster than kq_dequantize and a matmul */
+int kq_dequant_mul_mat(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m, int64_t stride_x,
+                       void* y, int64_t stride_y, void* stream);
+int kq_dequant_mul_mat_status(int* status, int clear);
+
 /* Embedding lookup: out[i, :] = the dequantized row row_ids[i] of the [n, k] weight tensor, i < count - the
  * torch.index_select + ggml_dequantize pair of the reference's GGUF embedding (quantization/vocal_embeds.py:38-55) in
  * one kernel, without the gathered copy of the wire rows.  f32_math = 0: arithmetic of kq_dequantize; f32_math = 1, for

@@ -24,7 +24,7 @@ EXPORTS = (
     "kq_get_option", "kq_prepare_q8", "kq_mul_mat_prepared", "kq_read_status", "kq_mul_mat_vec_a8_static",
     "kq_p2p_allgather", "kq_read_status_static", "kq_debug_copy_window", "kq_prepare_q8_rmsnorm", "kq_prepare_q8_swiglu",
     "kq_p2p_allgather_2d", "kq_mul_mat_prepared_gather", "kq_moe_a8_vec", "kq_moe_a8", "kq_moe_block_size", "kq_dequantize_rows", "kq_wait_arrival", "kq_arrival_status",
-    "kq_moe_project", "kq_moe_align", "kq_moe_combine",
+    "kq_dequant_mul_mat_supported", "kq_dequant_mul_mat_preferred", "kq_dequant_mul_mat", "kq_dequant_mul_mat_status", "kq_moe_project", "kq_moe_align", "kq_moe_combine",
 )
 
 
@@ -72,6 +72,9 @@ def _load() -> ctypes.CDLL:
     lib.kq_moe_a8.argtypes = [vp, i32, i64, i64, i64, vp, i32, i64, i64, vp, i64, vp, vp, i32, vp, i32, i64, vp, sz, vp]
     lib.kq_moe_block_size.argtypes = [i32]
     lib.kq_dequantize_rows.argtypes = [vp, i32, i64, i64, vp, i64, vp, i32, i32, vp]
+    lib.kq_dequant_mul_mat.argtypes = [vp, i32, i64, i64, vp, i32, i64, i64, vp, i64, vp]
+    lib.kq_dequant_mul_mat_preferred.argtypes = [i64, i64]
+    lib.kq_dequant_mul_mat_status.argtypes = [ctypes.POINTER(i32), i32]
     lib.kq_set_option.argtypes = [ctypes.c_char_p, i32]
     lib.kq_get_option.argtypes = [ctypes.c_char_p, ctypes.POINTER(i32)]
     return lib

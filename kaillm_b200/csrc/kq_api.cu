@@ -337,6 +337,36 @@ int kq_dequantize_rows(const void* W, int type, int64_t n, int64_t k, const int6
   return launch_dequantize(W, type, count * k, out, out_dtype, (cudaStream_t)stream, row_ids, k, n, f32_math != 0);
 }
 
+int kq_dequant_mul_mat_supported(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m, int64_t stride_x) {
+  return n > 0 && m > 0 && k > 0 && n <= 0x7fffffff / 2 && k <= (1 << 24) && m <= (1 << 20) && (dtype == KQ_F16 || dtype == KQ_BF16) &&
+         stride_x >= k && dense_mm_supported(W, type, k, x, stride_x);
+}
+
+// One launch reads the weights once per 256 tokens, about 2.2 (IQ3_S) to 2.6 us per 256-weight column and wave of 128-row
+// tiles; dequantize + matmul costs about 1 us per million weights.  So the tiles have to fill most of their waves: us, two
+// steps / one kernel at 16 tokens: IQ3_S 17408x5120 88 / 47, 4096x4096 22 / 38, 5120x17408 95 / 145; IQ4_XS 89 / 54, 20 / 44, 95 / 171.
+int kq_dequant_mul_mat_preferred(int64_t n, int64_t m) {
+  const int64_t tok = m <= 64 ? 64 : m <= 128 ? 128 : 256, tiles = (n + 127) / 128 * ((m + tok - 1) / tok);
+  const int64_t sms = sm_count(), waves = (tiles + sms - 1) / sms;
+  return n >= 12288 * waves;
+}
+
+int kq_dequant_mul_mat(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m, int64_t stride_x, void* y,
+                       int64_t stride_y, void* stream) {
+  t_err[0] = 0;
+  if (!W || !x || !y || stride_y < n || (uintptr_t)y % 2) { set_error("kq_dequant_mul_mat: null or misaligned pointer, or stride_y < n"); return KQ_EINVAL; }
+  if (!kq_dequant_mul_mat_supported(W, type, n, k, x, dtype, m, stride_x)) {
+    set_error("kq_dequant_mul_mat: IQ3_S, IQ4_NL, IQ4_XS with fp16 or bf16 activations, k a multiple of 256, W and every row of x 16-byte aligned");
+    return KQ_EUNSUPPORTED;
+  }
+  return launch_dense_mm(W, type, n, k, x, dtype, m, stride_x, y, stride_y, (cudaStream_t)stream);
+}
+
+int kq_dequant_mul_mat_status(int* status, int clear) {
+  t_err[0] = 0;
+  return dense_mm_status(status, clear);
+}
+
 int kq_debug_group_dots(const void* W, int type, int64_t n, int64_t k, const void* x, int x_dtype, int64_t m,
                         int64_t stride_x, int32_t* dots, int32_t* sums, void* scratch, size_t scratch_bytes,
                         void* stream) {

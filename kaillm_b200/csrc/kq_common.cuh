@@ -294,6 +294,10 @@ bool gemm_tc_supported(const void* W, int type, int64_t n, int64_t k);
 bool gemm_tc_staged(int type);   // the format's wire bytes reach the unpacking threads through shared memory
 int launch_gemm_tc(const void* W, int type, int64_t n, int64_t k, const Q8Ptrs& P, int64_t m, void* y, int y_dtype,
                    int64_t stride_y, bool mmq, cudaStream_t st);
+bool dense_mm_supported(const void* W, int type, int64_t k, const void* x, int64_t stride_x);
+int launch_dense_mm(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m, int64_t stride_x, void* y,
+                    int64_t stride_y, cudaStream_t st);
+int dense_mm_status(int* status, int clear);
 int launch_dequantize(const void* W, int type, int64_t count, void* out, int out_dtype, cudaStream_t st,
                       const int64_t* ids = nullptr, int64_t k = 0, int64_t nrows = 0, int f32math = 0);
 

@@ -25,6 +25,8 @@
 //             "accumulators complete".
 //   TMEM: 256 accumulator columns (2 x 128) + an A ring of 2 slots x 128 columns; shared memory: a B ring of 5 steps x
 //   32 KB.  Every mbarrier wait is bounded; on give-up a status word is set, TMEM is released and the CTA returns.
+#include <type_traits>
+
 #include "kq_common.cuh"
 #include "kq_tma.cuh"
 
@@ -41,23 +43,24 @@ constexpr uint32_t TMEM_D = 0;                 // accumulators: 256 columns
 constexpr uint32_t TMEM_A = 256;               // A ring: 256 columns
 constexpr int W6_ROW = 232;                    // Q6_K: bytes per staged row (216-byte aligned window of a 210-byte block, padded)
 
-// Two tile shapes, same TMEM budget (256 accumulator columns + 256 columns of A ring):
-//   narrow  2 row tiles x 128 tokens: warp w unpacks for row tile w>>3, atom (w>>2)&1 of EVERY step; an unpacked
-//           weight meets 128 tokens.  For m <= 128.
-//   wide    1 row tile x 256 tokens (UMMA N = 256): the two groups of 8 warps take alternate K steps (group w>>3
-//           serves the steps of its parity), so an unpacked weight meets 256 tokens - half the unpacking
-//           instructions per flop, twice the activation bytes per flop (64 KB per step through a ring of 3).
-template <bool WIDE>
+// Tile shapes (TS), at most 256 accumulator columns + 256 columns of A ring:
+//   0 narrow  2 row tiles x 128 tokens: warp w unpacks for row tile w>>3, atom (w>>2)&1 of EVERY step; an unpacked
+//             weight meets 128 tokens.  IQ3_S and unstaged K at m <= 128.
+//   1..3 wide 1 row tile x 256 / 128 / 64 tokens (UMMA N): the two groups of 8 warps take alternate K steps (group w>>3
+//             serves the steps of its parity).  An unpacked weight meets every token of the tile, so the tile is as wide as
+//             m allows; the narrower tiles leave shared memory for a ring of weight columns.
+//             The q8_1 formats always take 256 tokens; 128 and 64 serve the dequantizing GEMM.
+// B ring: stages of AB swizzle atoms (64 k x BN tokens) each.
+template <int TS>
 struct Tile {
+  static constexpr bool WIDE = TS != 0;
   static constexpr int RT = WIDE ? 1 : 2;          // accumulators (row tiles) per CTA
-  static constexpr int BN = WIDE ? 256 : 128;      // tokens per CTA = UMMA N
+  static constexpr int BN = TS == 1 ? 256 : TS == 3 ? 64 : 128;      // tokens per CTA = UMMA N
   static constexpr int NA = WIDE ? 4 : 2;          // A ring slots
-  static constexpr int NB = WIDE ? 3 : 5;          // B ring stages
   static constexpr int SLOT = RT * 64;             // TMEM columns per A slot: row tile t, atom a at t * 64 + a * 32
-  static constexpr int B_STAGE = BN * KSTEP * 2;   // 32 / 64 KB
+  static constexpr int AB = TS <= 1 ? 2 : 1;       // atoms per B stage
+  static constexpr int B_STAGE = AB * BN * ATOM * 2;   // 8 / 16 / 32 / 64 KB
   static constexpr int A_ARRIVALS = WIDE ? DQ_WARPS / 2 : DQ_WARPS;
-  static constexpr int W4_STAGE = RT * BM * 144;   // Q4_K: one super-block column of the CTA's rows
-  static constexpr int W6_STAGE = RT * BM * W6_ROW;
 };
 constexpr long long GEMM_WAIT_LIMIT = 1ll << 28;
 
@@ -345,6 +348,10 @@ template <> struct Win<KQ_TYPE_Q8_0> { static constexpr bool ON = true; static c
 template <> struct Win<KQ_TYPE_Q4_0> { static constexpr bool ON = true; static constexpr int COLB = 144, PIECES = 9, SROW = 144, NG = 9; };
 // Q2_K blocks are 4-byte aligned (84 = 4 * 21): a block starts 0, 4, 8 or 12 bytes into its window of 6 pieces
 template <> struct Win<KQ_TYPE_Q2_K> { static constexpr bool ON = true; static constexpr int COLB = 84, PIECES = 6, SROW = 112, NG = 10; };
+// i-matrix formats.  IQ3_S blocks are 2-byte aligned (110 bytes), IQ4_XS blocks 8-byte aligned (136)
+template <> struct Win<KQ_TYPE_IQ3_S> { static constexpr bool ON = true; static constexpr int COLB = 110, PIECES = 8, SROW = 144, NG = 8; };
+template <> struct Win<KQ_TYPE_IQ4_NL> { static constexpr bool ON = true; static constexpr int COLB = 144, PIECES = 9, SROW = 144, NG = 9; };
+template <> struct Win<KQ_TYPE_IQ4_XS> { static constexpr bool ON = true; static constexpr int COLB = 136, PIECES = 9, SROW = 144, NG = 10; };
 
 // bytes (b0, b1) and (b2, b3) of `w`, each plus 1024, as fp16 pairs (the bytes land in the mantissas of 0x6400)
 __device__ __forceinline__ __half2 bytes01_plus1024(uint32_t w) { return bits_h2(__byte_perm(w, 0x64646464u, 0x4140)); }
@@ -387,7 +394,8 @@ __device__ __forceinline__ void dequant_q4_0_regs(const uint32_t (&g)[9], uint32
 // Q2_K atom a4 of a super-block: half h = a4 >> 1 (qs bytes 32h..32h+31 = g[1..8]), 2-bit fields 2 * (a4 & 1) and
 // 2 * (a4 & 1) + 1; g[0] = its four scale bytes (sc | mn << 4, one per 16 weights), g[9] = {d, dmin}.
 // Same fp16 operations as the scalar path: half(sc * q) exact, then d * that minus dmin * mn in the order `fma` selects.
-__device__ __forceinline__ void dequant_q2_k_regs(const uint32_t (&g)[10], int odd, int fma, uint32_t (&out)[32]) {
+template <int FMA>
+__device__ __forceinline__ void dequant_q2_k_mode(const uint32_t (&g)[10], int odd, uint32_t (&out)[32]) {
   const __half2 k1024 = __half2half2(__ushort_as_half(0x6400));
   const __half2 dm = bits_h2(g[9]);
   const __half2 d2 = __half2half2(__low2half(dm)), dmin2 = __half2half2(__high2half(dm));
@@ -398,41 +406,155 @@ __device__ __forceinline__ void dequant_q2_k_regs(const uint32_t (&g)[10], int o
     for (int hh = 0; hh < 2; ++hh) {               // 16 weights under one scale byte
       const uint32_t sb = (g[0] >> (8 * (2 * run + hh))) & 0xFFu;
       const __half2 sc2 = __half2half2(__int2half_rn((int)(sb & 15u))), mn2 = __half2half2(__int2half_rn((int)(sb >> 4)));
-      const __half2 mp2 = __hmul2_rn(dmin2, mn2);
+      const __half2 nmp2 = __hneg2(__hmul2_rn(dmin2, mn2));
+      const __half2 nbias = __hneg2(__hmul2_rn(k1024, sc2));   // exact: at most 15360
 #pragma unroll
       for (int w = 0; w < 4; ++w) {
         const uint32_t code = (g[1 + 4 * hh + w] >> sh) & 0x03030303u;
 #pragma unroll
         for (int q = 0; q < 2; ++q) {
-          const __half2 xq = __hmul2_rn(__hsub2(q ? bytes23_plus1024(code) : bytes01_plus1024(code), k1024), sc2);
+          // (1024 + code) * sc - 1024 * sc: exact, code * sc <= 45
+          const __half2 xq = __hfma2(q ? bytes23_plus1024(code) : bytes01_plus1024(code), sc2, nbias);
           __half2 r;
-          if (fma == 2) r = __hfma2(__hneg2(dmin2), mn2, __hmul2_rn(d2, xq));
-          else if (fma) r = __hfma2(d2, xq, __hneg2(mp2));
-          else r = __hsub2(__hmul2_rn(d2, xq), mp2);
+          if (FMA == 2) r = __hfma2(__hneg2(dmin2), mn2, __hmul2_rn(d2, xq));
+          else if (FMA == 1) r = __hfma2(d2, xq, nmp2);
+          else r = __hadd2_rn(__hmul2_rn(d2, xq), nmp2);
           out[16 * run + 8 * hh + 2 * w + q] = h2_bits(r);
         }
       }
     }
   }
 }
+__device__ __forceinline__ void dequant_q2_k_regs(const uint32_t (&g)[10], int odd, int fma, uint32_t (&out)[32]) {
+  if (fma == 2) dequant_q2_k_mode<2>(g, odd, out);
+  else if (fma) dequant_q2_k_mode<1>(g, odd, out);
+  else dequant_q2_k_mode<0>(g, odd, out);
+}
+
+// The i-matrix formats as ggml_dequantize forms them: fp32 product of scale and code value, one rounding to the operand type.
+template <typename T> __device__ __forceinline__ uint32_t pack2(float a, float b);
+template <> __device__ __forceinline__ uint32_t pack2<__half>(float a, float b) { return h2_bits(__floats2half2_rn(a, b)); }
+template <> __device__ __forceinline__ uint32_t pack2<__nv_bfloat16>(float a, float b) {
+  const __nv_bfloat162 v = __floats2bfloat162_rn(a, b);
+  return *reinterpret_cast<const uint32_t*>(&v);
+}
+
+// IQ3_S atom: g[0..3] = 16 index bytes, g[4..5] = 8 sign bytes, g[6] = two high-bit bytes | the scale byte << 16, g[7] = d.
+// A sub-block has eight magnitudes (level l < 7: 8l + 4, level 7: the codebook's top byte) times one scale: they are rounded
+// once each and kept as two byte tables, so that four weights are two byte permutes by the codebook entry (four level
+// nibbles in `sel`) and two more to interleave; the signs are then set in the packed words (rounding is symmetric).
+template <typename T>
+__device__ __forceinline__ void dequant_iq3s_regs(const uint32_t (&g)[8], const uint16_t* sel, uint32_t (&out)[32]) {
+  const float d = __half2float(__ushort_as_half((unsigned short)g[7]));
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const uint32_t s4 = (g[6] >> (16 + 4 * e)) & 15u, qh = (g[6] >> (8 * e)) & 255u;
+    const float dl = __fmul_rn(__fmul_rn(d, 0.5f + (float)s4), 0.5f);
+    uint32_t m[4];
+#pragma unroll
+    for (int i = 0; i < 4; ++i)
+      m[i] = pack2<T>(__fmul_rn(dl, (float)(16 * i + 4)), __fmul_rn(dl, i == 3 ? (float)KQ_IQ3S_TOP : (float)(16 * i + 12)));
+    const uint32_t l0 = __byte_perm(m[0], m[1], 0x6420), h0 = __byte_perm(m[0], m[1], 0x7531);
+    const uint32_t l1 = __byte_perm(m[2], m[3], 0x6420), h1 = __byte_perm(m[2], m[3], 0x7531);
+#pragma unroll
+    for (int il = 0; il < 4; ++il) {
+      const uint32_t q2 = (g[2 * e + (il >> 1)] >> (16 * (il & 1))) & 0xFFFFu;
+      const uint32_t s = (g[4 + e] >> (8 * il)) & 255u;
+      const uint32_t c0 = sel[(q2 & 255u) | ((qh << (8 - 2 * il)) & 256u)], c1 = sel[(q2 >> 8) | ((qh << (7 - 2 * il)) & 256u)];
+      const uint32_t a0 = __byte_perm(l0, l1, c0), b0 = __byte_perm(h0, h1, c0), a1 = __byte_perm(l0, l1, c1), b1 = __byte_perm(h0, h1, c1);
+      uint32_t* o = out + 16 * e + 4 * il;
+      o[0] = __byte_perm(a0, b0, 0x5140) ^ ((s * 0x40008000u) & 0x80008000u);   // sign bits 0, 1 -> bits 15, 31
+      o[1] = __byte_perm(a0, b0, 0x7362) ^ ((s * 0x10002000u) & 0x80008000u);
+      o[2] = __byte_perm(a1, b1, 0x5140) ^ ((s * 0x04000800u) & 0x80008000u);
+      o[3] = __byte_perm(a1, b1, 0x7362) ^ ((s * 0x01000200u) & 0x80008000u);
+    }
+  }
+}
+
+// four 4-bit indices -> four products d * code value, packed: the biased code byte lands in the mantissa of 2^23
+template <typename T>
+__device__ __forceinline__ void iq4_four(uint32_t idx, float d, uint32_t& o0, uint32_t& o1) {
+  const uint32_t kv = iq4nl_lookup(idx) ^ 0x80808080u;
+  float f[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[i] = __fmul_rn(d, __uint_as_float(__byte_perm(kv, 0x4B000000u, 0x7540 + i)) - 8388736.0f);
+  o0 = pack2<T>(f[0], f[1]); o1 = pack2<T>(f[2], f[3]);
+}
+// IQ4_NL atom: two 18-byte blocks {d, 16 nibble bytes} = g[0..8]; the second block's bytes are word aligned
+template <typename T>
+__device__ __forceinline__ void dequant_iq4nl_regs(const uint32_t (&g)[9], uint32_t (&out)[32]) {
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const float d = __half2float(__ushort_as_half((unsigned short)(e ? g[4] >> 16 : g[0])));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = e ? g[5 + j] : __byte_perm(g[j], g[j + 1], 0x5432);
+      iq4_four<T>(w & 0x0F0F0F0Fu, d, out[16 * e + 2 * j], out[16 * e + 2 * j + 1]);
+      iq4_four<T>((w >> 4) & 0x0F0F0F0Fu, d, out[16 * e + 8 + 2 * j], out[16 * e + 8 + 2 * j + 1]);
+    }
+  }
+}
+// IQ4_XS atom a4: g[0] = {d, high scale bits}, g[1] = the four low-scale bytes, g[2..9] = the 32 nibble bytes
+template <typename T>
+__device__ __forceinline__ void dequant_iq4xs_regs(const uint32_t (&g)[10], int a4, uint32_t (&out)[32]) {
+  const float dh = __half2float(__ushort_as_half((unsigned short)g[0]));
+#pragma unroll
+  for (int e = 0; e < 2; ++e) {
+    const int ib = 2 * a4 + e;
+    const int ls = (int)(((g[1] >> (8 * a4 + 4 * e)) & 15u) | (((g[0] >> (16 + 2 * ib)) & 3u) << 4));
+    const float d = __fmul_rn(dh, (float)(ls - 32));
+#pragma unroll
+    for (int j = 0; j < 4; ++j) {
+      const uint32_t w = g[2 + 4 * e + j];
+      iq4_four<T>(w & 0x0F0F0F0Fu, d, out[16 * e + 2 * j], out[16 * e + 2 * j + 1]);
+      iq4_four<T>((w >> 4) & 0x0F0F0F0Fu, d, out[16 * e + 8 + 2 * j], out[16 * e + 8 + 2 * j + 1]);
+    }
+  }
+}
+
+// a bounded wait ran out in a call that has no scratch (kq_dequant_mul_mat): sticky, read by kq_dequant_mul_mat_status
+__device__ int g_dense_status = 0;
 
 // ------------------------------------------------------------------------------------------------ kernel
-template <int QT, bool CORR, typename OutT, bool WIDE>
+// DENSE: the activations are the caller's own 16-bit tensor (type OutT, B operand by TMA straight from it) and the weights
+// are rounded to the same type, i.e. what ggml_dequantize + matmul multiplies, without the dense weight matrix in memory.
+// Ring of staged weight columns (NW buffers of WSTAGE bytes) and ring of activation atoms (NB): what fits 227 KB.
+//   One buffer costs two barriers of the unpacking warps and the latency of the copies per column; with two or more the
+//   copies run NW - 1 columns ahead and one barrier is left.
+template <int QT, int TS>
+struct Rings {
+  using T = Tile<TS>;
+  static constexpr int WSTAGE = QT == KQ_TYPE_Q4_K ? T::RT * BM * 144 : QT == KQ_TYPE_Q6_K ? T::RT * BM * W6_ROW
+                                : (T::WIDE && Win<QT>::ON) ? BM * Win<QT>::SROW : 0;
+  static constexpr int HEAD = QT == KQ_TYPE_IQ3_S ? 4096 : 1024;      // barriers (+ IQ3_S codebook)
+  static constexpr int LIMIT = 227 * 1024;
+  static constexpr int NB = TS == 0 ? 5 : TS == 1 ? 3 : TS == 2 ? 6 : 8;
+  static constexpr int FIT = WSTAGE ? (LIMIT - HEAD - NB * T::B_STAGE) / WSTAGE : 0;
+  static constexpr int NW = !WSTAGE ? 0 : !T::WIDE ? 1 : FIT > 6 ? 6 : FIT;
+  static constexpr int SMEM = NB * T::B_STAGE + HEAD + NW * WSTAGE;
+  static_assert(NB <= 8 && SMEM <= LIMIT && (!WSTAGE || FIT >= 1), "shared memory budget");
+};
+
+template <int QT, bool CORR, typename OutT, int TS, bool DENSE>
 __global__ void __launch_bounds__(GEMM_THREADS, 1)
 gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, const __grid_constant__ CUtensorMap smap) {
   using F = Fmt<QT>;
-  using T = Tile<WIDE>;
-  constexpr int RT = T::RT, BN = T::BN, NA = T::NA, NB = T::NB, A_SLOT_COLS = T::SLOT, B_STAGE_BYTES = T::B_STAGE;
+  using T = Tile<TS>;
+  using R = Rings<QT, TS>;
+  constexpr bool WIDE = T::WIDE;
+  constexpr int RT = T::RT, BN = T::BN, NA = T::NA, NB = R::NB, A_SLOT_COLS = T::SLOT, B_STAGE_BYTES = T::B_STAGE;
+  constexpr int NW = R::NW, WSTAGE = R::WSTAGE, AB = T::AB;
   extern __shared__ __align__(1024) uint8_t smem[];
-  uint8_t* sB = smem;                                            // NB stages; each atom [BN rows x 128 B] swizzled
+  uint8_t* sB = smem;                                            // NB stages of AB atoms [BN rows x 128 B] swizzled
   uint64_t* bars = reinterpret_cast<uint64_t*>(smem + NB * B_STAGE_BYTES);
   uint32_t* tmem_slot = reinterpret_cast<uint32_t*>(bars + 26);
   volatile int* s_abort = reinterpret_cast<volatile int*>(bars + 27);
   uint32_t* s_grid = reinterpret_cast<uint32_t*>(bars + 32);     // IQ3_S codebook (2 KB)
-  uint8_t* sW = smem + NB * B_STAGE_BYTES + (QT == KQ_TYPE_IQ3_S ? 4096 : 1024);                // staged super-block column of the CTA's rows (Q4_K 144 B, Q6_K 232 B per row)
+  uint16_t* s_sel = reinterpret_cast<uint16_t*>(s_grid + 512);   // IQ3_S: the codebook as level nibbles (1 KB)
+  uint8_t* sW = smem + NB * B_STAGE_BYTES + R::HEAD;             // NW staged super-block columns of the CTA's rows
   const uint32_t bar_bfull = smem_u32(bars), bar_bempty = smem_u32(bars + 8), bar_afull = smem_u32(bars + 16),
                  bar_aempty = smem_u32(bars + 20), bar_dfull = smem_u32(bars + 24);
-  static_assert(NB <= 8 && NA <= 4, "barrier layout");
+  static_assert(NA <= 4, "barrier layout");
 
   const int tid = threadIdx.x, warp = tid >> 5, lane = tid & 31;
   const int row_tile = blockIdx.x / p.ntok_tiles, tok_tile = blockIdx.x % p.ntok_tiles;
@@ -448,7 +570,11 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
     asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
   }
   if constexpr (QT == KQ_TYPE_IQ3_S) {
-    for (int i = tid; i < 512; i += GEMM_THREADS) s_grid[i] = iq3s_expand(c_iq3s_codes_g[i], KQ_IQ3S_TOP);
+    for (int i = tid; i < 512; i += GEMM_THREADS) {
+      const uint32_t c = c_iq3s_codes_g[i];
+      s_grid[i] = iq3s_expand(c, KQ_IQ3S_TOP);
+      s_sel[i] = (uint16_t)((c & 7u) | ((c & 0x38u) << 1) | ((c & 0x1C0u) << 2) | ((c & 0xE00u) << 3));
+    }
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(TMEM_COLS));
@@ -462,15 +588,16 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
   if (warp == DQ_WARPS) {
     // -------------------------------------------------------------------------- activation loader (TMA)
     if (lane == 0) {
-      for (int s = 0; s < nsteps; ++s) {
-        const int buf = s % NB, fill = s / NB;
+      for (int i = 0; i < 2 * nsteps / AB; ++i) {     // stage i: atoms i * AB ..
+        const int buf = i % NB, fill = i / NB;
         if (fill > 0 && !mbar_wait(bar_bempty + 8 * buf, (uint32_t)((fill - 1) & 1), s_abort)) break;
         mbar_expect_tx(bar_bfull + 8 * buf, B_STAGE_BYTES);
 #pragma unroll
-        for (int a = 0; a < KSTEP / ATOM; ++a) {
+        for (int a = 0; a < AB; ++a) {
           const uint32_t dst = smem_u32(sB + buf * B_STAGE_BYTES + a * (BN * 128));
-          if (s < nmain) tma_load_2d(dst, &xmap, s * KSTEP + a * ATOM, tok_tile * BN, bar_bfull + 8 * buf);
-          else tma_load_2d(dst, &smap, (s - nmain) * KSTEP + a * ATOM, tok_tile * BN, bar_bfull + 8 * buf);
+          const int atom = i * AB + a;
+          if (atom < 2 * nmain) tma_load_2d(dst, &xmap, atom * ATOM, tok_tile * BN, bar_bfull + 8 * buf);
+          else tma_load_2d(dst, &smap, (atom - 2 * nmain) * ATOM, tok_tile * BN, bar_bfull + 8 * buf);
         }
       }
     }
@@ -478,18 +605,23 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
     // -------------------------------------------------------------------------- MMA issuer
     if (lane == 0) {
       // instruction descriptor: D = f32, A = B = f16, both K-major, N >> 3 at bit 17, M >> 4 at bit 24
-      const uint32_t idesc = (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
+      // (bf16 operands: formats 1 in bits 7 and 10)
+      constexpr uint32_t kinds = DENSE && std::is_same<OutT, __nv_bfloat16>::value ? (1u << 7) | (1u << 10) : 0u;
+      const uint32_t idesc = kinds | (1u << 4) | ((uint32_t)(BN >> 3) << 17) | ((uint32_t)(BM >> 4) << 24);
       bool ok = true;
       for (int s = 0; s < nsteps && ok; ++s) {
-        const int ab = s % NA, bb = s % NB;
-        ok = mbar_wait(bar_bfull + 8 * bb, (uint32_t)((s / NB) & 1), s_abort) &&
-             mbar_wait(bar_afull + 8 * ab, (uint32_t)((s / NA) & 1), s_abort);
-        if (!ok) break;
-        asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+        const int ab = s % NA;
 #pragma unroll
         for (int a = 0; a < KSTEP / ATOM; ++a) {
+          const int bi = (2 * s + a) / AB, bb = bi % NB;
+          if (AB == 1 || a == 0) {
+            ok = mbar_wait(bar_bfull + 8 * bb, (uint32_t)((bi / NB) & 1), s_abort) &&
+                 (a > 0 || mbar_wait(bar_afull + 8 * ab, (uint32_t)((s / NA) & 1), s_abort));
+            if (!ok) break;
+            asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+          }
           // shared-memory descriptor: addr >> 4, LBO (unused with swizzle), SBO = 1024 B, version 1, 128-byte swizzle
-          const uint32_t baddr = smem_u32(sB + bb * B_STAGE_BYTES + a * (BN * 128));
+          const uint32_t baddr = smem_u32(sB + bb * B_STAGE_BYTES + (AB == 2 ? a : 0) * (BN * 128));
           const uint64_t bdesc = (uint64_t)((baddr & 0x3FFFF) >> 4) | (1ull << 16) | ((uint64_t)(1024 >> 4) << 32) |
                                  (1ull << 46) | (2ull << 61);
 #pragma unroll
@@ -504,10 +636,11 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
                   ::"r"(tbase + TMEM_D + t * BN), "r"(ta), "l"(bdesc + (uint64_t)((kk * 32) >> 4)), "r"(idesc), "r"(accum) : "memory");
             }
           }
+          // completion of everything issued so far frees the B stage (and, after the second atom, the step's A slot)
+          if (AB == 1 || a == 1)
+            asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_bempty + 8 * bb) : "memory");
         }
-        // completion of everything issued so far frees this step's A slot and B stage
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_aempty + 8 * ab) : "memory");
-        asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_bempty + 8 * bb) : "memory");
+        if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_aempty + 8 * ab) : "memory");
       }
       if (ok) asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar_dfull) : "memory");
     }
@@ -564,7 +697,10 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
     }
     const bool holds_last_row = (row_tile + 1) * RT * BM >= p.n;   // rows past n are clamped to row n - 1
     const int last_sblk = p.k / 256 - 1;
-    auto stage_block = [&](int sblk) {                          // issue the copies of super-block column sblk
+    const int last_col = (nmain + 1) / 2 - 1;
+    auto stage_block = [&](int sblk) {                          // issue the copies of super-block column sblk into its ring buffer
+      if (sblk > last_col) { asm volatile("cp.async.commit_group;" ::: "memory"); return; }   // nothing left: keep the group count
+      const uint32_t wbuf = (uint32_t)(sblk % (NW > 0 ? NW : 1)) * (uint32_t)WSTAGE;
       if constexpr (WINQ) {
         // The window of the LAST column of the LAST row may reach a few bytes past the tensor (Q2_K: up to 12).  Only a
         // CTA that holds that row, and only there, takes the careful path, where a piece reads just the bytes that
@@ -577,14 +713,14 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
           if (csrc[i]) {
             const uint8_t* src = reinterpret_cast<const uint8_t*>((uintptr_t)(csrc[i] + col) & ~(uintptr_t)15) + ((cdst[i] >> 24) << 4);
             const uint32_t have = (!careful || src + 16 <= wend) ? 16u : (src < wend ? (uint32_t)(wend - src) : 0u);
-            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(cdst[i] & 0xFFFFFFu), "l"(src), "r"(have) : "memory");
+            asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"((cdst[i] & 0xFFFFFFu) + wbuf), "l"(src), "r"(have) : "memory");
           }
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
       if constexpr (QT == KQ_TYPE_Q4_K) {
 #pragma unroll
         for (int i = 0; i < NCHUNK; ++i)
-          if (csrc[i]) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(cdst[i]), "l"(csrc[i] + (size_t)sblk * 144) : "memory");
+          if (csrc[i]) asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(cdst[i] + wbuf), "l"(csrc[i] + (size_t)sblk * 144) : "memory");
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
       if constexpr (QT == KQ_TYPE_Q6_K) {
@@ -599,19 +735,31 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
             if (csrc[i]) {
               const uint8_t* src = csrc[i] + col;
               const uint32_t have = src + 8 <= wend ? 8u : (src < wend ? (uint32_t)(wend - src) : 0u);
-              asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(cdst[i]), "l"(src), "r"(have) : "memory");
+              asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;" ::"r"(cdst[i] + wbuf), "l"(src), "r"(have) : "memory");
             }
         } else {
 #pragma unroll
           for (int i = 0; i < NCHUNK; ++i)
-            if (csrc[i]) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(cdst[i]), "l"(csrc[i] + col) : "memory");
+            if (csrc[i]) asm volatile("cp.async.ca.shared.global [%0], [%1], 8;" ::"r"(cdst[i] + wbuf), "l"(csrc[i] + col) : "memory");
         }
         asm volatile("cp.async.commit_group;" ::: "memory");
       }
     };
     auto dq_barrier = [&]() { asm volatile("bar.sync 1, %0;" ::"n"(DQ_THREADS) : "memory"); };
     uint32_t gq[WN::NG] = {};                         // window formats: the words of the thread's atom
-    if (QT == KQ_TYPE_Q4_K || st6 || stw) stage_block(0);
+    // a new column: its copies have landed for everyone (and, with two buffers or more, everyone has pulled the column
+    // before it, whose buffer is refilled next)
+    auto column_landed = [&]() {
+      asm volatile("cp.async.wait_group %0;" ::"n"(NW >= 2 ? NW - 2 : 0) : "memory");
+      dq_barrier();
+    };
+    auto column_pulled = [&](int col) {
+      if (NW >= 2) { stage_block(col + NW - 1); return; }
+      dq_barrier();                                   // everyone has its bytes: the only buffer may be refilled
+      if (col + 1 <= last_col) stage_block(col + 1);
+    };
+    if (QT == KQ_TYPE_Q4_K || st6 || stw)
+      for (int i = 0; i < (NW >= 2 ? NW - 1 : 1); ++i) stage_block(i);
     // narrow: one iteration per step.  wide: one iteration per PAIR of steps (= super-block column); the thread
     // unpacks for step 2 * it + grp only, but takes part in the staging of every column.
     const int niter = WIDE ? (nsteps + 1) / 2 : nsteps;
@@ -625,9 +773,8 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
       uint32_t v[32];
       if constexpr (QT == KQ_TYPE_Q4_K) {
         if (new_col) {
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-          dq_barrier();                               // the whole column has landed
-          const uint8_t* mine = sW + (t * BM + rloc) * 144;
+          column_landed();
+          const uint8_t* mine = sW + (col % (NW > 0 ? NW : 1)) * WSTAGE + (t * BM + rloc) * 144;
           hdr4 = *reinterpret_cast<const uint4*>(mine);
 #pragma unroll
           for (int e = 0; e < NE; ++e) {              // narrow: atoms `half` (this step) and `half + 2` (next step); wide: atom 2 * grp + half
@@ -635,16 +782,14 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
             qa[e][0] = *reinterpret_cast<const uint4*>(mine + 16 + 32 * a4);
             qa[e][1] = *reinterpret_cast<const uint4*>(mine + 32 + 32 * a4);
           }
-          dq_barrier();                               // everyone has its bytes: the buffer may be refilled
-          if (2 * (col + 1) < nmain) stage_block(col + 1);
+          column_pulled(col);
         }
       }
       if constexpr (QT == KQ_TYPE_Q6_K) {
         if (st6 && new_col) {
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-          dq_barrier();
+          column_landed();
           const uint32_t off = (uint32_t)(((size_t)col * 210) & 7);        // where the block starts inside its window
-          const uint8_t* mine = sW + (t * BM + rloc) * W6_ROW + off;
+          const uint8_t* mine = sW + (col % (NW > 0 ? NW : 1)) * WSTAGE + (t * BM + rloc) * W6_ROW + off;
           const uint32_t fsh = ((uint32_t)(uintptr_t)mine & 2u) << 3;      // 0 or 16: the same for all rows
           auto words = [&](const uint8_t* ptr, uint32_t* dst, int n) {     // n 32-bit words from a 2-byte aligned address
             const uint32_t* q = reinterpret_cast<const uint32_t*>((uintptr_t)ptr & ~(uintptr_t)3);
@@ -660,28 +805,38 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
             words(mine + 192 + 8 * ip + 4 * half, &q6s[e], 1);
           }
           q6d = *reinterpret_cast<const __half*>(mine + 208);
-          dq_barrier();
-          if (2 * (col + 1) < nmain) stage_block(col + 1);
+          column_pulled(col);
         }
       }
       if constexpr (WINQ) {
         if (stw && new_col) {
-          asm volatile("cp.async.wait_group 0;" ::: "memory");
-          dq_barrier();
+          column_landed();
           const uint32_t off = (uint32_t)((uintptr_t)(wrow + (size_t)col * WN::COLB) & 15);   // where the column starts inside its window
-          const uint8_t* mine = sW + rloc * WN::SROW + off;
+          const uint8_t* mine = sW + (col % (NW > 0 ? NW : 1)) * WSTAGE + rloc * WN::SROW + off;
           const int a4 = 2 * grp + half;
           if constexpr (QT == KQ_TYPE_Q2_K) {
             gq[0] = *reinterpret_cast<const uint32_t*>(mine + 4 * a4);
 #pragma unroll
             for (int i = 0; i < 8; ++i) gq[1 + i] = *reinterpret_cast<const uint32_t*>(mine + 16 + 32 * grp + 4 * i);
             gq[9] = *reinterpret_cast<const uint32_t*>(mine + 80);
+          } else if constexpr (QT == KQ_TYPE_IQ3_S) {
+            auto u16 = [&](int at) { return (uint32_t)*reinterpret_cast<const uint16_t*>(mine + at); };
+#pragma unroll
+            for (int i = 0; i < 4; ++i) gq[i] = u16(2 + 16 * a4 + 4 * i) | (u16(4 + 16 * a4 + 4 * i) << 16);
+#pragma unroll
+            for (int i = 0; i < 2; ++i) gq[4 + i] = u16(74 + 8 * a4 + 4 * i) | (u16(76 + 8 * a4 + 4 * i) << 16);
+            gq[6] = u16(66 + 2 * a4) | ((uint32_t)mine[106 + a4] << 16);
+            gq[7] = u16(0);
+          } else if constexpr (QT == KQ_TYPE_IQ4_XS) {
+            gq[0] = *reinterpret_cast<const uint32_t*>(mine);
+            gq[1] = *reinterpret_cast<const uint32_t*>(mine + 4);
+#pragma unroll
+            for (int i = 0; i < 8; ++i) gq[2 + i] = *reinterpret_cast<const uint32_t*>(mine + 8 + 32 * a4 + 4 * i);
           } else {
 #pragma unroll
             for (int i = 0; i < WN::NG; ++i) gq[i] = *reinterpret_cast<const uint32_t*>(mine + (WN::COLB / 4) * a4 + 4 * i);
           }
-          dq_barrier();
-          if (2 * (col + 1) < nmain) stage_block(col + 1);
+          column_pulled(col);
         }
       }
       if (s >= nsteps) continue;                      // wide, odd number of steps: nothing left for this group
@@ -700,7 +855,11 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
           if constexpr (WINQ && QT == KQ_TYPE_Q8_0) dequant_q8_0_regs(gq, v);
           if constexpr (WINQ && QT == KQ_TYPE_Q4_0) dequant_q4_0_regs(gq, v);
           if constexpr (WINQ && QT == KQ_TYPE_Q2_K) dequant_q2_k_regs(gq, half, p.half_fma, v);
-        } else {
+          using OpT = typename std::conditional<DENSE, OutT, __half>::type;   // operand type
+          if constexpr (WINQ && QT == KQ_TYPE_IQ3_S) dequant_iq3s_regs<OpT>(gq, s_sel, v);
+          if constexpr (WINQ && QT == KQ_TYPE_IQ4_NL) dequant_iq4nl_regs<OpT>(gq, v);
+          if constexpr (WINQ && QT == KQ_TYPE_IQ4_XS) dequant_iq4xs_regs<OpT>(gq, 2 * grp + half, v);
+        } else if constexpr (!DENSE) {
           const uint8_t* blk = F::BLK >= 256 ? wrow + (size_t)(ga / ATOMS_PER_BLK) * F::BYTES
                                              : wrow + (size_t)ga * 2 * F::BYTES;
           dequant_atom<QT, CORR>(blk, F::BLK >= 256 ? (ga % ATOMS_PER_BLK) : 0, s_grid, p.half_fma, pre, v);
@@ -718,14 +877,15 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
         if (lane == 0) mbar_arrive(bar_afull + 8 * ab);
       }
     }
-    // -------------------------------------------------------------------------- epilogue: warp w takes the 64
-    // accumulator columns [64 * (w >> 2), +64) of its 32 lanes (narrow: that is its own row tile's accumulator)
+    // -------------------------------------------------------------------------- epilogue: the four warps of a lane quarter
+    // share the accumulator columns, EC each (narrow: 64, which is a warp's own row tile's accumulator)
     if (ok && mbar_wait(bar_dfull, 0, s_abort)) {
       asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
       OutT* y = reinterpret_cast<OutT*>(p.y);
-      const int cbase = (warp >> 2) * 64;
+      constexpr int EC = RT * BN >= 128 ? RT * BN / 4 : 32;
+      const int cbase = (warp >> 2) * EC;
 #pragma unroll 1
-      for (int c0 = cbase; c0 < cbase + 64; c0 += 32) {
+      for (int c0 = cbase; c0 < cbase + EC && c0 < RT * BN; c0 += 32) {
         uint32_t r[32];
         tmem_ld32(tbase + TMEM_D + lane_base + c0, r);
 #pragma unroll
@@ -736,7 +896,7 @@ gemm_tc_kernel(const GemmParams p, const __grid_constant__ CUtensorMap xmap, con
       }
     }
   }
-  if (*s_abort && tid == 0) atomicExch(p.status, 16);
+  if (*s_abort && tid == 0) atomicExch(DENSE ? &g_dense_status : p.status, 16);
   asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
   __syncthreads();
   if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tbase), "r"(TMEM_COLS));
@@ -757,13 +917,10 @@ __global__ void __launch_bounds__(256) q4_0_coef_kernel(const uint8_t* __restric
 
 // ------------------------------------------------------------------------------------------------ host
 
-template <int QT, bool CORR, typename OutT, bool WIDE>
+template <int QT, bool CORR, typename OutT, int TS, bool DENSE = false>
 int launch(const GemmParams& p, const CUtensorMap& map, const CUtensorMap& smap, int grid, cudaStream_t st) {
-  using T = Tile<WIDE>;
-  auto kern = gemm_tc_kernel<QT, CORR, OutT, WIDE>;
-  constexpr int WSTAGE = QT == KQ_TYPE_Q4_K ? T::W4_STAGE : QT == KQ_TYPE_Q6_K ? T::W6_STAGE : (WIDE && Win<QT>::ON) ? BM * Win<QT>::SROW : 0;
-  constexpr int smem = T::NB * T::B_STAGE + (QT == KQ_TYPE_IQ3_S ? 4096 : 1024) + WSTAGE;   // barriers (+ IQ3_S codebook), then the weight stage
-  static_assert(smem <= 227 * 1024, "shared memory budget");
+  auto kern = gemm_tc_kernel<QT, CORR, OutT, TS, DENSE>;
+  constexpr int smem = Rings<QT, TS>::SMEM;
   static DeviceOnce attr_set;   // the attribute belongs to the (function, device) pair
   if (attr_set.first_time()) {
     KQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
@@ -775,12 +932,21 @@ int launch(const GemmParams& p, const CUtensorMap& map, const CUtensorMap& smap,
   return KQ_OK;
 }
 
+template <int QT, typename OutT>
+int launch_dense(const GemmParams& p, const CUtensorMap& map, int grid, int ts, cudaStream_t st) {
+  switch (ts) {
+    case 1: return launch<QT, false, OutT, 1, true>(p, map, map, grid, st);
+    case 2: return launch<QT, false, OutT, 2, true>(p, map, map, grid, st);
+    default: return launch<QT, false, OutT, 3, true>(p, map, map, grid, st);
+  }
+}
+
 template <int QT, bool CORR>
 int launch_out(const GemmParams& p, const CUtensorMap& map, const CUtensorMap& smap, int grid, int y_dtype, bool wide, cudaStream_t st) {
   switch (y_dtype) {
-    case KQ_F32: return wide ? launch<QT, CORR, float, true>(p, map, smap, grid, st) : launch<QT, CORR, float, false>(p, map, smap, grid, st);
-    case KQ_F16: return wide ? launch<QT, CORR, __half, true>(p, map, smap, grid, st) : launch<QT, CORR, __half, false>(p, map, smap, grid, st);
-    case KQ_BF16: return wide ? launch<QT, CORR, __nv_bfloat16, true>(p, map, smap, grid, st) : launch<QT, CORR, __nv_bfloat16, false>(p, map, smap, grid, st);
+    case KQ_F32: return wide ? launch<QT, CORR, float, 1>(p, map, smap, grid, st) : launch<QT, CORR, float, 0>(p, map, smap, grid, st);
+    case KQ_F16: return wide ? launch<QT, CORR, __half, 1>(p, map, smap, grid, st) : launch<QT, CORR, __half, 0>(p, map, smap, grid, st);
+    case KQ_BF16: return wide ? launch<QT, CORR, __nv_bfloat16, 1>(p, map, smap, grid, st) : launch<QT, CORR, __nv_bfloat16, 0>(p, map, smap, grid, st);
   }
   set_error("unsupported output dtype %d", y_dtype);
   return KQ_EUNSUPPORTED;
@@ -814,7 +980,7 @@ int launch_gemm_tc(const void* W, int type, int64_t n, int64_t k, const Q8Ptrs& 
   // more than 128 tokens come, and at every m for the staged formats (measured at 96 tokens: Q4_K 17408x5120 39.8
   // against 58.3 us, Q6_K 17408x5120 53.4 against 142 us - unpacking, not the tensor pipe, is what a step costs)
   const bool wide = options().gemm_wide == 2 || (options().gemm_wide == 1 && (m > 128 || gemm_tc_staged(type)));
-  const int BN = wide ? Tile<true>::BN : Tile<false>::BN, RT = wide ? Tile<true>::RT : Tile<false>::RT;
+  const int BN = wide ? Tile<1>::BN : Tile<0>::BN, RT = wide ? Tile<1>::RT : Tile<0>::RT;
   const cuuint32_t box[2] = {ATOM, (cuuint32_t)BN};
   const cuuint32_t estr[2] = {1, 1};
   const CUresult r = enc(&map, CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)P.xh, gdim, gstr, box, estr,
@@ -856,6 +1022,47 @@ int launch_gemm_tc(const void* W, int type, int64_t n, int64_t k, const Q8Ptrs& 
     case KQ_TYPE_IQ3_S: return launch_out<KQ_TYPE_IQ3_S, false>(p, map, smap, grid, y_dtype, wide, st);
   }
   return KQ_EUNSUPPORTED;
+}
+
+// y = x @ dequantize(W)^T for the i-matrix formats, x fp16 or bf16 (the weights are rounded to x's type)
+bool dense_mm_supported(const void* W, int type, int64_t k, const void* x, int64_t stride_x) {
+  return (type == KQ_TYPE_IQ3_S || type == KQ_TYPE_IQ4_NL || type == KQ_TYPE_IQ4_XS) && k % 256 == 0 && ((uintptr_t)W % 16) == 0 &&
+         ((uintptr_t)x % 16) == 0 && stride_x % 8 == 0 && encode_fn() != nullptr;
+}
+
+int launch_dense_mm(const void* W, int type, int64_t n, int64_t k, const void* x, int dtype, int64_t m, int64_t stride_x, void* y,
+                    int64_t stride_y, cudaStream_t st) {
+  int blk = 1, bytes = 1;
+  type_geometry(type, &blk, &bytes);
+  const int ts = m <= 64 ? 3 : m <= 128 ? 2 : 1, BN = ts == 1 ? 256 : ts == 3 ? 64 : 128;
+  CUtensorMap map;
+  const cuuint64_t gdim[2] = {(cuuint64_t)k, (cuuint64_t)m};
+  const cuuint64_t gstr[1] = {(cuuint64_t)stride_x * 2};
+  const cuuint32_t box[2] = {ATOM, (cuuint32_t)BN}, estr[2] = {1, 1};
+  const CUresult r = encode_fn()(&map, dtype == KQ_BF16 ? CU_TENSOR_MAP_DATA_TYPE_BFLOAT16 : CU_TENSOR_MAP_DATA_TYPE_FLOAT16, 2, (void*)x,
+                                 gdim, gstr, box, estr, CU_TENSOR_MAP_INTERLEAVE_NONE, CU_TENSOR_MAP_SWIZZLE_128B,
+                                 CU_TENSOR_MAP_L2_PROMOTION_L2_256B, CU_TENSOR_MAP_FLOAT_OOB_FILL_NONE);
+  if (r != CUDA_SUCCESS) { set_error("dequantizing GEMM: cuTensorMapEncodeTiled failed (%d)", (int)r); return KQ_ECUDA; }
+  GemmParams p = {};
+  p.nb32 = (int)(k / 32); p.W = (const uint8_t*)W; p.rowbytes = k / blk * bytes; p.n = (int)n; p.k = (int)k; p.m = (int)m;
+  p.ntok_tiles = (int)((m + BN - 1) / BN); p.y = y; p.stride_y = stride_y; p.half_fma = options().half_fma; p.stagew = 1;
+  const int64_t grid = (n + BM - 1) / BM * p.ntok_tiles;
+  if (grid > 0x7fffffff) { set_error("dequantizing GEMM: too many tiles"); return KQ_ELIMIT; }
+  const bool bf = dtype == KQ_BF16;
+  switch (type) {
+    case KQ_TYPE_IQ3_S: return bf ? launch_dense<KQ_TYPE_IQ3_S, __nv_bfloat16>(p, map, (int)grid, ts, st) : launch_dense<KQ_TYPE_IQ3_S, __half>(p, map, (int)grid, ts, st);
+    case KQ_TYPE_IQ4_NL: return bf ? launch_dense<KQ_TYPE_IQ4_NL, __nv_bfloat16>(p, map, (int)grid, ts, st) : launch_dense<KQ_TYPE_IQ4_NL, __half>(p, map, (int)grid, ts, st);
+    case KQ_TYPE_IQ4_XS: return bf ? launch_dense<KQ_TYPE_IQ4_XS, __nv_bfloat16>(p, map, (int)grid, ts, st) : launch_dense<KQ_TYPE_IQ4_XS, __half>(p, map, (int)grid, ts, st);
+  }
+  return KQ_EUNSUPPORTED;
+}
+
+int dense_mm_status(int* status, int clear) {
+  int v = 0;
+  KQ_CUDA_TRY(cudaMemcpyFromSymbol(&v, g_dense_status, sizeof(int)));
+  if (status) *status = v;
+  if (clear && v) { const int z = 0; KQ_CUDA_TRY(cudaMemcpyToSymbol(g_dense_status, &z, sizeof(int))); }
+  return KQ_OK;
 }
 
 }  // namespace kq

@@ -89,6 +89,30 @@ at::Tensor ggml_dequantize(const at::Tensor& W, int64_t type, c10::SymInt m_, c1
   return DW;
 }
 
+// X @ dequantize(W)^T: one kernel where it covers the call, otherwise the two steps
+at::Tensor ggml_dequant_mul_mat(const at::Tensor& W, const at::Tensor& X, int64_t type, c10::SymInt row_) {
+  const char* fn = "ggml_dequant_mul_mat";
+  const int64_t row = row_.expect_int();
+  int blk = 0, bytes = 0;
+  TORCH_CHECK(kq_block_geometry((int)type, &blk, &bytes) == KQ_OK, fn, ": ", kq_last_error());
+  TORCH_CHECK(W.dim() == 2, fn, ": W must be 2-D");
+  const bool half = X.scalar_type() == at::kHalf || X.scalar_type() == at::kBFloat16;
+  if (half && W.is_cuda() && X.is_cuda() && W.get_device() == X.get_device() && W.scalar_type() == at::kByte && W.is_contiguous() &&
+      X.dim() == 2 && X.stride(1) == 1 && W.size(0) == row && X.size(1) % blk == 0 && W.size(1) == X.size(1) / blk * bytes) {
+    const int64_t m = X.size(0), k = X.size(1);
+    const int xdt = kq_dtype_of(X.scalar_type(), fn);
+    if (kq_dequant_mul_mat_preferred(row, m) && kq_dequant_mul_mat_supported(W.data_ptr(), (int)type, row, k, X.data_ptr(), xdt, m, X.stride(0))) {
+      const c10::cuda::CUDAGuard guard(X.device());
+      at::Tensor Y = at::empty({m, row}, X.options());
+      auto stream = at::cuda::getCurrentCUDAStream(X.get_device()).stream();
+      TORCH_CHECK(kq_dequant_mul_mat(W.data_ptr(), (int)type, row, k, X.data_ptr(), xdt, m, X.stride(0), Y.data_ptr(), Y.stride(0),
+                                     (void*)stream) == KQ_OK, fn, ": ", kq_last_error());
+      return Y;
+    }
+  }
+  return at::matmul(X, ggml_dequantize(W, type, c10::SymInt(row), c10::SymInt(W.size(1) / bytes * blk), X.scalar_type()).t());
+}
+
 // W: [E, row, row bytes] (or any contiguous uint8 tensor holding E matrices back to back)
 at::Tensor moe_impl(bool block, const at::Tensor& X, const at::Tensor& W, const at::Tensor& ids, const at::Tensor* expert_ids,
                     const at::Tensor* num_post_padded, int64_t type, int64_t row, int64_t top_k, int64_t tokens) {
@@ -208,6 +232,7 @@ TORCH_LIBRARY(_C_gguf, ops) {
   ops.def("ggml_dequantize(Tensor W, int type, SymInt m, SymInt n, ScalarType? dtype) -> Tensor");
   ops.def("ggml_mul_mat_vec_a8(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("ggml_mul_mat_a8(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
+  ops.def("ggml_dequant_mul_mat(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def(
       "ggml_moe_a8(Tensor X, Tensor W, Tensor sorted_token_ids, Tensor expert_ids, Tensor "
       "num_tokens_post_padded, int type, SymInt row, SymInt top_k, SymInt tokens) -> Tensor");
@@ -222,6 +247,7 @@ TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_dequantize", &ggml_dequantize);
   ops.impl("ggml_mul_mat_vec_a8", &ggml_mul_mat_vec_a8);
   ops.impl("ggml_mul_mat_a8", &ggml_mul_mat_a8);
+  ops.impl("ggml_dequant_mul_mat", &ggml_dequant_mul_mat);
   ops.impl("ggml_moe_a8", &ggml_moe_a8);
   ops.impl("ggml_moe_a8_vec", &ggml_moe_a8_vec);
   ops.impl("fused_moe_swiglu", &fused_moe_swiglu);

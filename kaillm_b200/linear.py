@@ -40,6 +40,8 @@ def fused_mul_mat_gguf(x: torch.Tensor, qweight: torch.Tensor, qweight_type: int
     if qweight_type in MMQ_QUANT_TYPES:
         return ops.ggml_mul_mat_a8(qweight, x, qweight_type, qweight.shape[0])
     if qweight_type in DEQUANT_TYPES:
+        if _plain(x):
+            return ops.ggml_dequant_mul_mat(qweight, x, qweight_type, qweight.shape[0])
         block_size, type_size = BLOCK[qweight_type]
         shape = (qweight.shape[0], qweight.shape[1] // type_size * block_size)
         weight = ops.ggml_dequantize(qweight, qweight_type, *shape, x.dtype)

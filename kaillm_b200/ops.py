@@ -47,6 +47,11 @@ def ggml_mul_mat_a8(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int)
     return torch.ops._C_gguf.ggml_mul_mat_a8(W, X, quant_type, row)
 
 
+def ggml_dequant_mul_mat(W: torch.Tensor, X: torch.Tensor, quant_type: int, row: int) -> torch.Tensor:
+    """X @ ggml_dequantize(W).T, fused where the kernel covers the call (no gradient: see linear.fused_mul_mat_gguf)."""
+    return torch.ops._C_gguf.ggml_dequant_mul_mat(W, X, quant_type, row)
+
+
 def ggml_moe_a8(X: torch.Tensor, W: torch.Tensor, sorted_token_ids: torch.Tensor, expert_ids: torch.Tensor,
                 num_tokens_post_padded: torch.Tensor, quant_type: int, row: int, top_k: int, tokens: int) -> torch.Tensor:
     """vllm_gguf_plugin/ops.py:211-246."""
