@@ -56,29 +56,19 @@ __device__ __forceinline__ void store8(OutT* dst, const __half2 (&h)[4]) {
   }
 }
 
-struct RowGather {
-  const int64_t* ids;   // nullptr: the blocks are taken in storage order
-  int64_t k, rowbytes, nrows;
-  int f32math;          // Q4_K / Q5_K / Q6_K: fp32 products as gguf-reader and the reference's embedding decoder form them
-};
+// four byte codes -> float(code - bias), exactly: a byte in the mantissa of 2^23
+__device__ __forceinline__ void codes_f32(uint32_t w, int bias, float (&f)[8], int at) {
+#pragma unroll
+  for (int i = 0; i < 4; ++i) f[at + i] = __uint_as_float(__byte_perm(w, 0x4B000000u, 0x7540 + i)) - (float)(8388608 + bias);
+}
 
 // eight consecutive weights starting at element e0
 template <int QT, typename OutT>
 __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64_t e0, OutT* __restrict__ out, int fma,
-                                            const RowGather& g, const uint32_t* s_grid) {
+                                            int f32math, const uint32_t* s_grid) {
+  // f32math: fp32 products for Q4_K / Q5_K / Q6_K, as gguf-reader and the reference's embedding decoder form them
   using F = Fmt<QT>;
   const uint8_t* b = W + (e0 / F::BLK) * F::BYTES;
-  if (g.ids != nullptr) {
-    // output row r is weight row ids[r] (an embedding lookup); a row index outside the tensor gives zeros
-    const int64_t r = e0 / g.k, src = g.ids[r];
-    if (src < 0 || src >= g.nrows) {
-      const uint4 z = make_uint4(0u, 0u, 0u, 0u);
-      reinterpret_cast<uint4*>(out + e0)[0] = z;
-      if constexpr (sizeof(OutT) == 4) reinterpret_cast<uint4*>(out + e0)[1] = z;
-      return;
-    }
-    b = W + src * g.rowbytes + ((e0 - r * g.k) / F::BLK) * F::BYTES;
-  }
   const int r0 = (int)(e0 % F::BLK);
   OutT res[8];
   if constexpr (QT == KQ_TYPE_Q4_0) {
@@ -141,7 +131,7 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
     else { sc = (q[jj + 4] & 15) | ((q[jj - 4] >> 6) << 4); mn = (q[jj + 4] >> 4) | ((q[jj] >> 6) << 4); }
     const __half d1 = __hmul_rn(dall, __int2half_rn(sc));
     const __half m1 = __hmul_rn(dmin, __int2half_rn(mn));
-    if (!g.f32math) {   // d1 * q - m1, two weights at a time
+    if (!f32math) {   // d1 * q - m1, two weights at a time
       const uint8_t* q8 = b + 16 + 32 * il + l0;
       const bool al4 = ((uintptr_t)q8 & 3) == 0;       // the tensor may start on a 2-byte boundary only
       const uint32_t r0w = al4 ? ld_u32(q8) : ld_u16x2(q8), r1w = al4 ? ld_u32(q8 + 4) : ld_u16x2(q8 + 4);
@@ -156,21 +146,22 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
       store8<OutT>(out + e0, h);
       return;
     }
+    {   // (d * sc) * q - dmin * m with every product and the difference rounded in fp32
+      const uint8_t* q8 = b + 16 + 32 * il + l0;
+      const bool al4 = ((uintptr_t)q8 & 3) == 0;
+      const uint32_t r0w = al4 ? ld_u32(q8) : ld_u16x2(q8), r1w = al4 ? ld_u32(q8 + 4) : ld_u16x2(q8 + 4);
+      float f[8];
+      codes_f32((r0w >> (4 * hi)) & 0x0F0F0F0Fu, 0, f, 0);
+      codes_f32((r1w >> (4 * hi)) & 0x0F0F0F0Fu, 0, f, 4);
+      const float ds = __fmul_rn(__half2float(dall), (float)sc), dm = __fmul_rn(__half2float(dmin), (float)mn);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int byte = b[16 + 32 * il + l0 + j];
-      const int qq = hi ? (byte >> 4) : (byte & 15);
-      if (g.f32math)   // (d * sc) * q - dmin * m with every product and the difference rounded in fp32
-        res[j] = from_f32<OutT>(__fsub_rn(__fmul_rn(__fmul_rn(__half2float(dall), (float)sc), (float)qq),
-                                          __fmul_rn(__half2float(dmin), (float)mn)));
-      else
-        res[j] = half_to_out<OutT>(mul_sub(d1, __int2half_rn(qq), m1, fma));
+      for (int j = 0; j < 8; ++j) res[j] = from_f32<OutT>(__fsub_rn(__fmul_rn(ds, f[j]), dm));
     }
   } else if constexpr (QT == KQ_TYPE_Q6_K) {
     const __half d = __ushort_as_half(*reinterpret_cast<const uint16_t*>(b + 208));
     const int ip = r0 >> 7, q4 = (r0 >> 5) & 3, l0 = r0 & 31;
     const int sc = (int8_t)b[192 + 8 * ip + 2 * q4 + (l0 >> 4)];
-    if (!g.f32math) {   // d * half(sc * (code - 32)): sc and code - 32 are exact in fp16, so half(sc) * half(code - 32) rounds once, like the conversion of the integer product
+    if (!f32math) {   // d * half(sc * (code - 32)): sc and code - 32 are exact in fp16, so half(sc) * half(code - 32) rounds once, like the conversion of the integer product
       const uint8_t* pl = b + 64 * ip + 32 * (q4 & 1) + l0;
       const uint8_t* ph = b + 128 + 32 * ip + l0;
       const uint32_t l0w = ld_u16x2(pl), l1w = ld_u16x2(pl + 4), h0w = ld_u16x2(ph), h1w = ld_u16x2(ph + 4);
@@ -189,14 +180,16 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
       store8<OutT>(out + e0, h);
       return;
     }
+    {   // (d * sc) * (code - 32), both products rounded in fp32
+      const uint8_t* pl = b + 64 * ip + 32 * (q4 & 1) + l0;
+      const uint8_t* ph = b + 128 + 32 * ip + l0;
+      const int sh = q4 < 2 ? 0 : 4;
+      const float ds = __fmul_rn(__half2float(d), (float)sc);
+      float f[8];
+      codes_f32(((ld_u16x2(pl) >> sh) & 0x0F0F0F0Fu) | (((ld_u16x2(ph) >> (2 * q4)) & 0x03030303u) << 4), 32, f, 0);
+      codes_f32(((ld_u16x2(pl + 4) >> sh) & 0x0F0F0F0Fu) | (((ld_u16x2(ph + 4) >> (2 * q4)) & 0x03030303u) << 4), 32, f, 4);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int lo = b[64 * ip + 32 * (q4 & 1) + l0 + j];
-      const int nib = (q4 < 2) ? (lo & 15) : (lo >> 4);
-      const int hb = (b[128 + 32 * ip + l0 + j] >> (2 * q4)) & 3;
-      const int code = (nib | (hb << 4)) - 32;
-      if (g.f32math) res[j] = from_f32<OutT>(__fmul_rn(__fmul_rn(__half2float(d), (float)sc), (float)code));   // (d * sc) * q
-      else res[j] = half_to_out<OutT>(__hmul_rn(d, __int2half_rn(sc * code)));
+      for (int j = 0; j < 8; ++j) res[j] = from_f32<OutT>(__fmul_rn(ds, f[j]));
     }
   } else if constexpr (QT == KQ_TYPE_IQ3_S) {
     const float dh = ld_h(b);
@@ -261,7 +254,7 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
     else { sc = (q[jj + 4] & 15) | ((q[jj - 4] >> 6) << 4); mn = (q[jj + 4] >> 4) | ((q[jj] >> 6) << 4); }
     const __half d1 = __hmul_rn(dall, __int2half_rn(sc));
     const __half m1 = __hmul_rn(dmin, __int2half_rn(mn));
-    if (!g.f32math) {   // as Q4_K, with the fifth bit of each code taken from qh
+    if (!f32math) {   // as Q4_K, with the fifth bit of each code taken from qh
       const uint8_t* q8 = b + 48 + 32 * il + l0;
       const uint8_t* qh8 = b + 16 + l0;
       const bool al4 = ((uintptr_t)q8 & 3) == 0;
@@ -279,15 +272,18 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
       store8<OutT>(out + e0, h);
       return;
     }
+    {   // as Q4_K, with the fifth bit of each code taken from qh
+      const uint8_t* q8 = b + 48 + 32 * il + l0;
+      const uint8_t* qh8 = b + 16 + l0;
+      const bool al4 = ((uintptr_t)q8 & 3) == 0;
+      const uint32_t r0w = al4 ? ld_u32(q8) : ld_u16x2(q8), r1w = al4 ? ld_u32(q8 + 4) : ld_u16x2(q8 + 4);
+      const uint32_t h0w = al4 ? ld_u32(qh8) : ld_u16x2(qh8), h1w = al4 ? ld_u32(qh8 + 4) : ld_u16x2(qh8 + 4);
+      float f[8];
+      codes_f32(((r0w >> (4 * hi)) & 0x0F0F0F0Fu) | (((h0w >> jj) & 0x01010101u) << 4), 0, f, 0);
+      codes_f32(((r1w >> (4 * hi)) & 0x0F0F0F0Fu) | (((h1w >> jj) & 0x01010101u) << 4), 0, f, 4);
+      const float ds = __fmul_rn(__half2float(dall), (float)sc), dm = __fmul_rn(__half2float(dmin), (float)mn);
 #pragma unroll
-    for (int j = 0; j < 8; ++j) {
-      const int byte = b[48 + 32 * il + l0 + j];
-      const int qq = (hi ? (byte >> 4) : (byte & 15)) + (((b[16 + l0 + j] >> jj) & 1) ? 16 : 0);
-      if (g.f32math)
-        res[j] = from_f32<OutT>(__fsub_rn(__fmul_rn(__fmul_rn(__half2float(dall), (float)sc), (float)qq),
-                                          __fmul_rn(__half2float(dmin), (float)mn)));
-      else
-        res[j] = half_to_out<OutT>(mul_sub(d1, __int2half_rn(qq), m1, fma));
+      for (int j = 0; j < 8; ++j) res[j] = from_f32<OutT>(__fsub_rn(__fmul_rn(ds, f[j]), dm));
     }
   } else if constexpr (QT == KQ_TYPE_IQ4_NL || QT == KQ_TYPE_IQ4_XS) {   // dequantize.cuh:401-437: fp32 d * code value
     float d = ld_h(b);
@@ -333,7 +329,7 @@ __device__ __forceinline__ void dequantize8(const uint8_t* __restrict__ W, int64
 // Grid-stride over chunks of eight weights (the launcher decides how many chunks a thread walks).
 template <int QT, typename OutT>
 __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restrict__ W, int64_t count,
-                                                         OutT* __restrict__ out, int fma, RowGather g) {
+                                                         OutT* __restrict__ out, int fma) {
   // IQ3_S: the expanded codebook in shared memory (lanes look up different entries: the constant cache would serialise them)
   __shared__ uint32_t s_grid[QT == KQ_TYPE_IQ3_S ? 512 : 1];
   if constexpr (QT == KQ_TYPE_IQ3_S) {
@@ -342,22 +338,67 @@ __global__ void __launch_bounds__(256) dequantize_kernel(const uint8_t* __restri
   }
   const int64_t step = (int64_t)gridDim.x * blockDim.x * 8;
   for (int64_t e0 = ((int64_t)blockIdx.x * blockDim.x + threadIdx.x) * 8; e0 < count; e0 += step)
-    dequantize8<QT, OutT>(W, e0, out, fma, g, s_grid);
+    dequantize8<QT, OutT>(W, e0, out, fma, 0, s_grid);
+}
+
+// An embedding lookup: output row r is weight row ids[r]; a row index outside the tensor gives zeros.  CTA = (output rows
+// blockIdx.x, + gridDim.x, ..; chunks of 8 weights from 256 * blockIdx.y): the row index is read once per CTA and no thread
+// divides by k.  Q6_K, 2048 rows x 5120 to bf16, whole call: 18.1 -> 10.2 us (the kernel was 11.7 us with one flat index per thread and
+// byte-wise fp32 products).
+template <int QT, typename OutT>
+__global__ void __launch_bounds__(256) dequantize_rows_kernel(const uint8_t* __restrict__ W, int64_t rowbytes, int64_t nrows, int64_t k,
+                                                              const int64_t* __restrict__ ids, int64_t rows, OutT* __restrict__ out,
+                                                              int fma, int f32math) {
+  __shared__ uint32_t s_grid[QT == KQ_TYPE_IQ3_S ? 512 : 1];
+  if constexpr (QT == KQ_TYPE_IQ3_S) {
+    for (int i = threadIdx.x; i < 512; i += blockDim.x) s_grid[i] = iq3s_expand(c_iq3s_codes_dq[i], KQ_IQ3S_TOP);
+    __syncthreads();
+  }
+  const int64_t e0 = ((int64_t)blockIdx.y * 256 + threadIdx.x) * 8;
+  if (e0 >= k) return;
+  for (int64_t r = blockIdx.x; r < rows; r += gridDim.x) {
+    const int64_t src = __ldg(ids + r);
+    OutT* o = out + r * k;
+    if (src < 0 || src >= nrows) {
+      const uint4 z = make_uint4(0u, 0u, 0u, 0u);
+      reinterpret_cast<uint4*>(o + e0)[0] = z;
+      if constexpr (sizeof(OutT) == 4) reinterpret_cast<uint4*>(o + e0)[1] = z;
+    } else {
+      dequantize8<QT, OutT>(W + src * rowbytes, e0, o, fma, f32math, s_grid);
+    }
+  }
+}
+
+struct RowGather {
+  const int64_t* ids;   // nullptr: the blocks are taken in storage order
+  int64_t k, rowbytes, nrows;
+  int f32math;
+};
+
+template <int QT, typename OutT>
+static void run_typed(const void* W, int64_t count, OutT* out, int fma, cudaStream_t st, const RowGather& g) {
+  // IQ3_S fills its codebook once per CTA: few CTAs that walk many chunks (rows); the other formats run best with one chunk per thread
+  constexpr bool BOOK = QT == KQ_TYPE_IQ3_S;
+  if (g.ids != nullptr) {
+    const int64_t rows = count / g.k, gy = (g.k / 8 + 255) / 256;
+    int64_t gx = BOOK ? ((int64_t)sm_count() * 16 + gy - 1) / gy : (int64_t)0x7fffffff;
+    if (gx > rows) gx = rows;
+    dequantize_rows_kernel<QT, OutT><<<dim3((unsigned)gx, (unsigned)gy), 256, 0, st>>>((const uint8_t*)W, g.rowbytes, g.nrows, g.k, g.ids, rows, out, fma, g.f32math);
+    return;
+  }
+  int64_t blocks = (count / 8 + 255) / 256;
+  const int64_t cap = BOOK ? (int64_t)sm_count() * 16 : (int64_t)0x7fffffff;
+  if (blocks > cap) blocks = cap;
+  dequantize_kernel<QT, OutT><<<(unsigned)blocks, 256, 0, st>>>((const uint8_t*)W, count, out, fma);
 }
 
 template <int QT>
 static int run(const void* W, int64_t count, void* out, int out_dtype, int fma, cudaStream_t st, const RowGather& g) {
-  const int64_t threads = count / 8;
-  int64_t blocks = (threads + 255) / 256;
-  // IQ3_S fills its codebook once per CTA: few CTAs that walk many chunks; the other formats run best with one chunk per thread
-  const int64_t cap = QT == KQ_TYPE_IQ3_S ? (int64_t)sm_count() * 16 : (int64_t)0x7fffffff;
-  if (blocks > cap) blocks = cap;
-  const unsigned grid = (unsigned)blocks;
-  if (grid == 0) return KQ_OK;
+  if (count / 8 == 0) return KQ_OK;
   switch (out_dtype) {
-    case KQ_F16: dequantize_kernel<QT, __half><<<grid, 256, 0, st>>>((const uint8_t*)W, count, (__half*)out, fma, g); break;
-    case KQ_BF16: dequantize_kernel<QT, __nv_bfloat16><<<grid, 256, 0, st>>>((const uint8_t*)W, count, (__nv_bfloat16*)out, fma, g); break;
-    case KQ_F32: dequantize_kernel<QT, float><<<grid, 256, 0, st>>>((const uint8_t*)W, count, (float*)out, fma, g); break;
+    case KQ_F16: run_typed<QT, __half>(W, count, (__half*)out, fma, st, g); break;
+    case KQ_BF16: run_typed<QT, __nv_bfloat16>(W, count, (__nv_bfloat16*)out, fma, st, g); break;
+    case KQ_F32: run_typed<QT, float>(W, count, (float*)out, fma, st, g); break;
     default: set_error("unsupported output dtype %d", out_dtype); return KQ_EUNSUPPORTED;
   }
   options().launches += 1;

@@ -113,6 +113,26 @@ at::Tensor ggml_dequant_mul_mat(const at::Tensor& W, const at::Tensor& X, int64_
   return at::matmul(X, ggml_dequantize(W, type, c10::SymInt(row), c10::SymInt(W.size(1) / bytes * blk), X.scalar_type()).t());
 }
 
+// rows `ids` (any shape) of the [n, row bytes] table W, dequantized: [*ids.shape, k]
+at::Tensor ggml_dequantize_rows(const at::Tensor& W, const at::Tensor& ids, int64_t type, int64_t k, at::ScalarType dtype, bool f32_math) {
+  const char* fn = "ggml_dequantize_rows";
+  check_weight(W, fn);
+  TORCH_CHECK(W.dim() == 2 && ids.is_cuda() && ids.get_device() == W.get_device(), fn, ": W must be 2-D and the ids on its device");
+  const int odt = kq_dtype_of(dtype, fn);
+  int blk = 0, bytes = 0;
+  TORCH_CHECK(kq_block_geometry((int)type, &blk, &bytes) == KQ_OK, fn, ": ", kq_last_error());
+  TORCH_CHECK(k > 0 && k % blk == 0 && W.size(1) == k / blk * bytes, fn, ": rows of W do not hold k=", k, " weights");
+  const c10::cuda::CUDAGuard guard(W.device());
+  const at::Tensor flat = ids.to(at::kLong).contiguous();
+  auto shape = ids.sizes().vec();
+  shape.push_back(k);
+  at::Tensor out = at::empty(shape, W.options().dtype(dtype));
+  const int rc = kq_dequantize_rows(W.data_ptr(), (int)type, W.size(0), k, flat.data_ptr<int64_t>(), flat.numel(), out.data_ptr(), odt,
+                                    f32_math, (void*)at::cuda::getCurrentCUDAStream(W.get_device()).stream());
+  TORCH_CHECK(rc == KQ_OK, fn, ": ", kq_last_error());
+  return out;
+}
+
 // W: [E, row, row bytes] (or any contiguous uint8 tensor holding E matrices back to back)
 at::Tensor moe_impl(bool block, const at::Tensor& X, const at::Tensor& W, const at::Tensor& ids, const at::Tensor* expert_ids,
                     const at::Tensor* num_post_padded, int64_t type, int64_t row, int64_t top_k, int64_t tokens) {
@@ -233,6 +253,7 @@ TORCH_LIBRARY(_C_gguf, ops) {
   ops.def("ggml_mul_mat_vec_a8(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("ggml_mul_mat_a8(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("ggml_dequant_mul_mat(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
+  ops.def("ggml_dequantize_rows(Tensor W, Tensor ids, int type, int k, ScalarType dtype, bool f32_math) -> Tensor");
   ops.def(
       "ggml_moe_a8(Tensor X, Tensor W, Tensor sorted_token_ids, Tensor expert_ids, Tensor "
       "num_tokens_post_padded, int type, SymInt row, SymInt top_k, SymInt tokens) -> Tensor");
@@ -248,6 +269,7 @@ TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_mul_mat_vec_a8", &ggml_mul_mat_vec_a8);
   ops.impl("ggml_mul_mat_a8", &ggml_mul_mat_a8);
   ops.impl("ggml_dequant_mul_mat", &ggml_dequant_mul_mat);
+  ops.impl("ggml_dequantize_rows", &ggml_dequantize_rows);
   ops.impl("ggml_moe_a8", &ggml_moe_a8);
   ops.impl("ggml_moe_a8_vec", &ggml_moe_a8_vec);
   ops.impl("fused_moe_swiglu", &fused_moe_swiglu);

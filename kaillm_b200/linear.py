@@ -88,12 +88,15 @@ def apply_gguf_embedding(x: torch.Tensor, qweight: torch.Tensor, qweight_type: i
     reads the selected rows in place (kq_dequantize_rows).  Q4_K / Q5_K / Q6_K are reconstructed with fp32 products, as
     the reference does for exactly these three formats (vocal_embeds.py:43-50); the others with ggml_dequantize's fp16
     arithmetic."""
-    from . import capi
     if qweight_type in UNQUANTIZED_TYPES:
         return torch.embedding(qweight, x)
     if qweight_type in DEQUANT_TYPES:
         block_size, type_size = BLOCK[qweight_type]
         assert hidden_size == qweight.shape[1] // type_size * block_size
+        if x.is_cuda and qweight.is_cuda and x.device == qweight.device and qweight.dtype == torch.uint8 and qweight.is_contiguous():
+            return ops.ggml_dequantize_rows(qweight, x, qweight_type, hidden_size, dtype or torch.float16,
+                                            qweight_type in F32_MATH_EMBEDDING_TYPES)
+        from . import capi
         return capi.dequantize_rows(qweight, qweight_type, hidden_size, x, dtype or torch.float16,
                                     f32_math=qweight_type in F32_MATH_EMBEDDING_TYPES)
     raise NotImplementedError(f"Unsupported GGUF quantization type: {qweight_type}")

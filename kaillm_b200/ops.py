@@ -52,6 +52,11 @@ def ggml_dequant_mul_mat(W: torch.Tensor, X: torch.Tensor, quant_type: int, row:
     return torch.ops._C_gguf.ggml_dequant_mul_mat(W, X, quant_type, row)
 
 
+def ggml_dequantize_rows(W: torch.Tensor, ids: torch.Tensor, quant_type: int, k: int, dtype: torch.dtype, f32_math: bool) -> torch.Tensor:
+    """Rows `ids` of the table W, dequantized (kq_dequantize_rows): [*ids.shape, k]."""
+    return torch.ops._C_gguf.ggml_dequantize_rows(W, ids, quant_type, k, dtype, f32_math)
+
+
 def ggml_moe_a8(X: torch.Tensor, W: torch.Tensor, sorted_token_ids: torch.Tensor, expert_ids: torch.Tensor,
                 num_tokens_post_padded: torch.Tensor, quant_type: int, row: int, top_k: int, tokens: int) -> torch.Tensor:
     """vllm_gguf_plugin/ops.py:211-246."""
