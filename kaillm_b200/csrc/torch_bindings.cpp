@@ -11,6 +11,8 @@
 //     (vllm_gguf_plugin/ops.py:110-175), but raise: they are outside this library's scope.
 #include <Python.h>
 
+#include <algorithm>
+
 #include <ATen/ATen.h>
 #include <ATen/cuda/CUDAContext.h>
 #include <ATen/cuda/CUDAEvent.h>
@@ -67,6 +69,45 @@ at::Tensor ggml_mul_mat_vec_a8(const at::Tensor& W, const at::Tensor& X, int64_t
 
 at::Tensor ggml_mul_mat_a8(const at::Tensor& W, const at::Tensor& X, int64_t type, c10::SymInt row) {
   return mul_mat_impl(true, W, X, type, row.expect_int());
+}
+
+// Projections of different types over the same activations (q/k/v of a mixed-type file): one quantization, every shard's
+// kernel writes its own columns of the merged output.  mmq[i]: which of the two ops shard i is.
+at::Tensor ggml_mul_mat_merged(at::TensorList Ws, const at::Tensor& X, at::IntArrayRef types, at::IntArrayRef mmq) {
+  const char* fn = "ggml_mul_mat_merged";
+  TORCH_CHECK(!Ws.empty() && Ws.size() == types.size() && Ws.size() == mmq.size(), fn, ": one type and flavour per shard");
+  TORCH_CHECK(X.is_cuda() && X.dim() == 2 && X.stride(1) == 1, fn, ": X must be a 2-D CUDA tensor, contiguous along its last dimension");
+  const int64_t m = X.size(0), k = X.size(1);
+  const int xdt = kq_dtype_of(X.scalar_type(), fn);
+  int64_t total = 0, widest = 0;
+  size_t ws = 0;
+  for (size_t i = 0; i < Ws.size(); ++i) {
+    const at::Tensor& W = Ws[i];
+    check_weight(W, fn);
+    int blk = 0, bytes = 0;
+    TORCH_CHECK(kq_block_geometry((int)types[i], &blk, &bytes) == KQ_OK, fn, ": ", kq_last_error());
+    TORCH_CHECK(W.dim() == 2 && W.get_device() == X.get_device(), fn, ": W must be 2-D and on X's device");
+    TORCH_CHECK(k % blk == 0 && W.size(1) == k / blk * bytes, fn, ": a shard does not hold rows of K=", k);
+    total += W.size(0);
+    widest = std::max(widest, W.size(0));
+  }
+  for (size_t i = 0; i < Ws.size(); ++i) ws = std::max(ws, kq_workspace_bytes((int)types[i], m, widest, k));
+  const c10::cuda::CUDAGuard guard(X.device());
+  at::Tensor Y = at::empty({m, total}, X.options());
+  if (m == 0 || total == 0) return Y;
+  at::Tensor scratch = at::empty({(int64_t)ws}, X.options().dtype(at::kByte));
+  void* stream = (void*)at::cuda::getCurrentCUDAStream(X.get_device()).stream();
+  TORCH_CHECK(kq_prepare_q8((int)types[0], widest, k, X.data_ptr(), xdt, m, X.stride(0), scratch.data_ptr(), ws, 0, stream) == KQ_OK, fn, ": ", kq_last_error());
+  int64_t col = 0;
+  for (size_t i = 0; i < Ws.size(); ++i) {
+    const int64_t n = Ws[i].size(0);
+    if (n == 0) continue;
+    void* y = static_cast<char*>(Y.data_ptr()) + col * (int64_t)Y.element_size();
+    TORCH_CHECK(kq_mul_mat_prepared(Ws[i].data_ptr(), (int)types[i], n, k, m, y, xdt, total, (int)mmq[i], scratch.data_ptr(), ws, stream) == KQ_OK,
+                fn, ": ", kq_last_error());
+    col += n;
+  }
+  return Y;
 }
 
 at::Tensor ggml_dequantize(const at::Tensor& W, int64_t type, c10::SymInt m_, c10::SymInt n_,
@@ -254,6 +295,7 @@ TORCH_LIBRARY(_C_gguf, ops) {
   ops.def("ggml_mul_mat_a8(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("ggml_dequant_mul_mat(Tensor W, Tensor X, int type, SymInt row) -> Tensor");
   ops.def("ggml_dequantize_rows(Tensor W, Tensor ids, int type, int k, ScalarType dtype, bool f32_math) -> Tensor");
+  ops.def("ggml_mul_mat_merged(Tensor[] W, Tensor X, int[] types, int[] mmq) -> Tensor");
   ops.def(
       "ggml_moe_a8(Tensor X, Tensor W, Tensor sorted_token_ids, Tensor expert_ids, Tensor "
       "num_tokens_post_padded, int type, SymInt row, SymInt top_k, SymInt tokens) -> Tensor");
@@ -270,6 +312,7 @@ TORCH_LIBRARY_IMPL(_C_gguf, CUDA, ops) {
   ops.impl("ggml_mul_mat_a8", &ggml_mul_mat_a8);
   ops.impl("ggml_dequant_mul_mat", &ggml_dequant_mul_mat);
   ops.impl("ggml_dequantize_rows", &ggml_dequantize_rows);
+  ops.impl("ggml_mul_mat_merged", &ggml_mul_mat_merged);
   ops.impl("ggml_moe_a8", &ggml_moe_a8);
   ops.impl("ggml_moe_a8_vec", &ggml_moe_a8_vec);
   ops.impl("fused_moe_swiglu", &fused_moe_swiglu);

@@ -28,11 +28,15 @@ def _plain(x: torch.Tensor) -> bool:
             and torch.autograd.forward_ad.unpack_dual(x).tangent is None)
 
 
-def fused_mul_mat_gguf(x: torch.Tensor, qweight: torch.Tensor, qweight_type: int) -> torch.Tensor:
+def _mmvq_safe(rows: int, qweight_type: int) -> int:
+    """Largest token count that goes to the mat-vec op."""
     if qweight_type in IMATRIX_QUANT_TYPES:
-        mmvq_safe = 8 if qweight.shape[0] > 5120 else 16
-    else:
-        mmvq_safe = 2 if qweight.shape[0] > 5120 else 6
+        return 8 if rows > 5120 else 16
+    return 2 if rows > 5120 else 6
+
+
+def fused_mul_mat_gguf(x: torch.Tensor, qweight: torch.Tensor, qweight_type: int) -> torch.Tensor:
+    mmvq_safe = _mmvq_safe(qweight.shape[0], qweight_type)
     if x.shape[0] == 0:
         return torch.empty(x.shape[0], qweight.shape[0], dtype=x.dtype, device=x.device)
     if x.shape[0] <= mmvq_safe and qweight_type in MMVQ_QUANT_TYPES:
@@ -65,11 +69,33 @@ class GGUFLinear:
         else:
             self.merged = None
 
+    def _one_preparation(self, x: torch.Tensor) -> list[int] | None:
+        """The op of every shard (0 mul_mat_vec, 1 mul_mat) where all of them multiply the same quantized activations: up to
+        80 tokens (above, one GEMM operand is quantized per call anyway) and no shard on the dequantize-and-multiply branch."""
+        if not (_plain(x) and 0 < x.shape[0] <= 80 and x.stride(1) == 1 and x.dtype in _FLOATS):
+            return None
+        flavours = []
+        for w, t in self.shards:
+            if t not in MMVQ_QUANT_TYPES or w.device != x.device or w.dtype != torch.uint8 or w.dim() != 2 or not w.is_contiguous():
+                return None
+            block_size, type_size = BLOCK[t]
+            if x.shape[1] % block_size or w.shape[1] != x.shape[1] // block_size * type_size:
+                return None
+            if x.shape[0] <= _mmvq_safe(w.shape[0], t):
+                flavours.append(0)
+            elif t in MMQ_QUANT_TYPES:
+                flavours.append(1)
+            else:
+                return None
+        return flavours
+
     def apply(self, x: torch.Tensor, bias: torch.Tensor | None = None) -> torch.Tensor:
         if self.merged is not None:
             out = fused_mul_mat_gguf(x, *self.merged)
         elif len(self.shards) == 1:
             out = fused_mul_mat_gguf(x, *self.shards[0])
+        elif (flavours := self._one_preparation(x)) is not None:
+            out = ops.ggml_mul_mat_merged([w for w, _ in self.shards], x, [t for _, t in self.shards], flavours)
         else:
             out = torch.cat([fused_mul_mat_gguf(x, w, t) for w, t in self.shards], dim=1)
         if bias is not None:

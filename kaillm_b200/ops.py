@@ -57,6 +57,11 @@ def ggml_dequantize_rows(W: torch.Tensor, ids: torch.Tensor, quant_type: int, k:
     return torch.ops._C_gguf.ggml_dequantize_rows(W, ids, quant_type, k, dtype, f32_math)
 
 
+def ggml_mul_mat_merged(Ws: list[torch.Tensor], X: torch.Tensor, quant_types: list[int], mmq: list[int]) -> torch.Tensor:
+    """Several projections of the same activations, quantized once: [m, sum of rows] (no gradient)."""
+    return torch.ops._C_gguf.ggml_mul_mat_merged(Ws, X, quant_types, mmq)
+
+
 def ggml_moe_a8(X: torch.Tensor, W: torch.Tensor, sorted_token_ids: torch.Tensor, expert_ids: torch.Tensor,
                 num_tokens_post_padded: torch.Tensor, quant_type: int, row: int, top_k: int, tokens: int) -> torch.Tensor:
     """vllm_gguf_plugin/ops.py:211-246."""
