@@ -7,8 +7,8 @@
 //   - outputs come from at::empty (the kernels write every element; the reference memsets with new_zeros);
 //   - an unsupported GGML type raises instead of silently returning zeros
 //     (reference: switch without default, csrc/gguf/gguf_kernel.cu:119-215);
-//   - the MoE ops are declared, so the unmodified Python wrapper can register its fake implementations
-//     (vllm_gguf_plugin/ops.py:110-175), but raise: they are outside this library's scope.
+//   - ops of this library's own beside the reference's six: ggml_dequant_mul_mat, ggml_dequantize_rows,
+//     ggml_mul_mat_merged, fused_moe_swiglu (no derivative: kaillm_b200/linear.py calls them for plain tensors only).
 #include <Python.h>
 
 #include <algorithm>
