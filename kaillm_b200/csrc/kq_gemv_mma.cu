@@ -452,7 +452,7 @@ __global__ void __launch_bounds__(ROW_THREADS, 1) gemv_rows_kernel(const RowPara
     const int swz = (lane >> 2) & 1;
     for (int sb = lane; sb < p.nsb; sb += 32) {
       SubBlock s;
-      decode_subblock<QT>(prow, sb, s_grid, s);
+      decode_subblock<QT, true>(prow, sb, s_grid, s);
 #pragma unroll
       for (int t = 0; t < MT; ++t) {
         const uint8_t* ap = sA + (size_t)t * p.a_stride + sb * 32;

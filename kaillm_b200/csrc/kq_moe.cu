@@ -223,23 +223,11 @@ __global__ void __launch_bounds__(256) moe_vec_smem_kernel(const MoeParams p) {
   }
 }
 
-// A sub-block out of a row staged in shared memory at its global address modulo 16.  Q8_0: nine aligned words and a funnel
-// shift instead of seventeen 16-bit loads; Q4_K (rows are 16-byte aligned): three 16-byte loads.
+// A sub-block out of a row staged in shared memory at its global address modulo 16; Q4_K (rows are 16-byte aligned): three
+// 16-byte loads.
 template <int QT>
 __device__ __forceinline__ void decode_staged(const uint8_t* row, int sb, const uint32_t* grid, SubBlock& o) {
-  if constexpr (QT == KQ_TYPE_Q8_0) {
-    const uint8_t* b = row + sb * 34;
-    o.wa[0] = ld_h(b); o.wa[1] = 0.f; o.wb[0] = 0.f; o.wb[1] = 0.f;
-    const uint32_t* w = reinterpret_cast<const uint32_t*>((uintptr_t)(b + 2) & ~(uintptr_t)3);
-    const uint32_t sh = ((uint32_t)(uintptr_t)(b + 2) & 2u) << 3;
-    uint32_t lo = w[0];
-#pragma unroll
-    for (int i = 0; i < 8; ++i) {        // the ninth word is the tail of this block or the start of what follows inside the stage
-      const uint32_t hi = w[i + 1];
-      o.v[i] = __funnelshift_r(lo, hi, sh);
-      lo = hi;
-    }
-  } else if constexpr (QT == KQ_TYPE_Q4_K) {
+  if constexpr (QT == KQ_TYPE_Q4_K) {
     const uint8_t* b = row + (sb >> 3) * 144;
     const int j = sb & 7;
     const uint4 h = *reinterpret_cast<const uint4*>(b);
@@ -255,7 +243,7 @@ __device__ __forceinline__ void decode_staged(const uint8_t* row, int sb, const 
 #pragma unroll
     for (int i = 0; i < 8; ++i) o.v[i] = (q[i] >> e4) & 0x0F0F0F0Fu;
   } else {
-    decode_subblock<QT>(row, sb, grid, o);
+    decode_subblock<QT, true>(row, sb, grid, o);
   }
 }
 
