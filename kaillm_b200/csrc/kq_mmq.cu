@@ -447,6 +447,7 @@ int launch_mmq_moe(const void* W, int type, int64_t experts, int64_t n, int64_t 
   mmq_params(p, W, type, experts, n, k, P, tokens, y, y_dtype, stride_y, rows);
   p.top_k = top_k; p.ids = ids; p.nslots = nslots; p.expert_ids = expert_ids; p.num_post_padded = num_post_padded;
   const int64_t nblocks = (nslots + KQ_MOE_BLOCK - 1) / KQ_MOE_BLOCK;
+  if (nblocks > 65535) { set_error("kq_moe_a8: more than 65535 blocks of sorted tokens"); return KQ_ELIMIT; }
   int64_t groups = (8ll * sm_count() + p.row_tiles - 1) / p.row_tiles;
   if (groups > nblocks) groups = nblocks;
   const unsigned grid = (unsigned)(groups * p.row_tiles);

@@ -36,7 +36,10 @@ def _mmvq_safe(rows: int, qweight_type: int) -> int:
 
 
 def fused_mul_mat_gguf(x: torch.Tensor, qweight: torch.Tensor, qweight_type: int) -> torch.Tensor:
-    mmvq_safe = _mmvq_safe(qweight.shape[0], qweight_type)
+    if qweight_type in IMATRIX_QUANT_TYPES:      # _mmvq_safe, written out: one token's call is bound by the host
+        mmvq_safe = 8 if qweight.shape[0] > 5120 else 16
+    else:
+        mmvq_safe = 2 if qweight.shape[0] > 5120 else 6
     if x.shape[0] == 0:
         return torch.empty(x.shape[0], qweight.shape[0], dtype=x.dtype, device=x.device)
     if x.shape[0] <= mmvq_safe and qweight_type in MMVQ_QUANT_TYPES:
