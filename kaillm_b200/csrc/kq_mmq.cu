@@ -5,8 +5,7 @@
 //
 // The row-streaming GEMV re-reads and re-decodes a weight for every 8 tokens, the old block op for every 8 slots.  Here a
 // weight is decoded once per 64 tokens (or slots of one expert): decoding is what bounded both (Q5_K 6144x5120 at 333
-// tokens was 42 passes).  The dots stay exact integers and the scales fp32, so the results have the GEMV's precision; fp16
-// operands on tcgen05 (kq_gemm_tc.cu) would not.
+// tokens was 42 passes).  The dots stay exact integers and the scales fp32; fp16 operands on tcgen05 (kq_gemm_tc.cu) would not.
 //
 //   CTA       8 warps; tile 128 (or 64) weight rows x up to 64 tokens; two CTAs share an SM, so that one decodes while
 //             another multiplies
@@ -17,10 +16,16 @@
 //             of the mma is the bit pattern of 12582912.0f, so the integer dot comes out as a float after one subtraction;
 //             two outputs per fp32x2 instruction
 //   tokens    codes, scales and min-term factors of a half column by cp.async, double buffered
+//   sums      The kernels this one replaces add a row in 32 lanes and a tree; one fp32 chain over K would lose against that
+//             (relative error against 64 bits, Q5_K, 1e-7: K = 512 1.07 against 0.63, 5120 3.05 against 0.81, 17408 6.1 against
+//             1.07).  So a chain ends after 8 sub-blocks (4 where K < 2048, 2 where K < 512: the shorter the row the better
+//             that tree) and is added to a sum and its correction in tensor memory, for which no register or shared memory
+//             is left: 0.57 / 0.69 / 0.72, and not above the replaced kernels' in any format from K = 256 on.  A
+//             sub-block's min term joins its dot before the chain.
 //
-// Measured (us, whole call, bf16 in and out, before -> now): Q5_K 6144x5120 at 64 / 100 / 333 tokens 144 / 229 / 755 -> 109 /
-// 110 / 197; Q3_K at 333 tokens 910 -> 207; the fused mixture-of-experts layer (32 experts, top 4, 2048/1408, Q4_K + Q8_0) at
-// 256 tokens 1068 -> 614.  What bounds it: latency of the half-column steps (load, decode, multiply behind barriers).
+// Measured (us, whole call, bf16 in and out, before -> now): Q5_K 6144x5120 at 64 / 100 / 333 tokens 144 / 229 / 755 -> 122 /
+// 123 / 219; Q3_K at 333 tokens 910 -> 229; the fused mixture-of-experts layer (32 experts, top 4, 2048/1408, Q4_K + Q8_0) at
+// 256 tokens 1057 -> 299.  What bounds it: latency of the half-column steps (load, decode, multiply behind barriers).
 //
 // Mixture of experts: a work item is a run of up to 8 consecutive 8-slot blocks of one expert; every CTA finds the items
 // from expert_ids itself and takes every gridDim-th of them.
@@ -47,9 +52,11 @@ template <int QT, int ROWS> struct Mq {
   static constexpr int RAW = ROWS * SROW, A = ROWS * STR, S = 4 * ROWS * NS * 4, B = MQ_TOK * STR;
   static constexpr int DS = MQ_TOK * 16, ZR = NG == 2 ? MQ_TOK * 32 : MQ_TOK * 16;   // raw ds / z pieces of a half column
   static constexpr int D = 4 * MQ_TOK * 4, Z = MIN ? 4 * NG * MQ_TOK * 4 : 0;
-  static constexpr int OFF_A = RAW, OFF_S = OFF_A + A, OFF_B = OFF_S + S, OFF_DS = OFF_B + 2 * B, OFF_ZR = OFF_DS + 2 * DS,
-                       OFF_D = OFF_ZR + (MIN ? 2 * ZR : 0), OFF_Z = OFF_D + D, OFF_TOK = OFF_Z + Z, SMEM = OFF_TOK + 2 * MQ_TOK * 4;
   static constexpr int WR = ROWS / 32, WN = MQ_WARPS / WR, NT = 8 / WN;   // warps over rows x tokens; 8-token tiles per warp
+  static constexpr int TCOLS = 2 * NT * 16;                        // tensor memory: two warps per lane quarter, {sum, correction} x 8 per tile
+  static constexpr int OFF_A = RAW, OFF_S = OFF_A + A, OFF_B = OFF_S + S, OFF_DS = OFF_B + 2 * B, OFF_ZR = OFF_DS + 2 * DS,
+                       OFF_D = OFF_ZR + (MIN ? 2 * ZR : 0), OFF_Z = OFF_D + D, OFF_TOK = OFF_Z + Z, SMEM = OFF_TOK + 2 * MQ_TOK * 4 + 16;   // 16: address of the tensor memory
+  static_assert(TCOLS >= 32 && (TCOLS & (TCOLS - 1)) == 0 && TCOLS <= 256, "two CTAs per SM share 512 columns");
   static_assert(OFF_TOK >= ROWS * 65 * 4, "the epilogue's transpose tile reuses the buffers");
 };
 
@@ -89,6 +96,19 @@ __device__ __forceinline__ void mq_mma_k16(int (&d)[4], uint32_t a0, uint32_t a1
       : "=r"(d[0]), "=r"(d[1]), "=r"(d[2]), "=r"(d[3])
       : "r"(a0), "r"(a1), "r"(b0), "r"(MQ_MAGIC));
 }
+// sixteen 32-bit words per lane of this warp's quarter of tensor memory
+__device__ __forceinline__ void mq_tmem_ld16(uint32_t at, uint32_t (&r)[16]) {
+  asm volatile("tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0,%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15}, [%16];\n\t"
+               "tcgen05.wait::ld.sync.aligned;"
+               : "=r"(r[0]), "=r"(r[1]), "=r"(r[2]), "=r"(r[3]), "=r"(r[4]), "=r"(r[5]), "=r"(r[6]), "=r"(r[7]), "=r"(r[8]), "=r"(r[9]),
+                 "=r"(r[10]), "=r"(r[11]), "=r"(r[12]), "=r"(r[13]), "=r"(r[14]), "=r"(r[15])
+               : "r"(at) : "memory");
+}
+__device__ __forceinline__ void mq_tmem_st16(uint32_t at, const uint32_t (&r)[16]) {
+  asm volatile("tcgen05.st.sync.aligned.32x32b.x16.b32 [%0], {%1,%2,%3,%4,%5,%6,%7,%8,%9,%10,%11,%12,%13,%14,%15,%16};"
+               ::"r"(at), "r"(r[0]), "r"(r[1]), "r"(r[2]), "r"(r[3]), "r"(r[4]), "r"(r[5]), "r"(r[6]), "r"(r[7]), "r"(r[8]), "r"(r[9]),
+                 "r"(r[10]), "r"(r[11]), "r"(r[12]), "r"(r[13]), "r"(r[14]), "r"(r[15]) : "memory");
+}
 __device__ __forceinline__ void mq_cp16(uint32_t dst, const void* src, uint32_t have) {
   asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;" ::"r"(dst), "l"(src), "r"(have) : "memory");
 }
@@ -122,7 +142,28 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
   const uint32_t smem_a = (uint32_t)__cvta_generic_to_shared(mq_smem);
   const int nhalf = (p.nsb + 3) >> 2, nb8 = p.kpad >> 5;
   const uint8_t* wend = p.W + p.wbytes;
-  pdl_trigger();
+  uint32_t* sTmem = reinterpret_cast<uint32_t*>(mq_smem + M::OFF_TOK + 2 * MQ_TOK * 4);
+  uint32_t tacc = 0;                                            // this warp's part of the tensor memory
+  // After pdl_wait() and before pdl_trigger(): a CTA never holds tensor memory while it waits for another kernel, and a kernel
+  // behind this one cannot take it first.
+  auto tmem_open = [&]() {
+    if (warp == 0) {
+      asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"((uint32_t)__cvta_generic_to_shared(sTmem)), "r"(M::TCOLS) : "memory");
+      asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;");
+    }
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    tacc = *sTmem + ((uint32_t)(warp & 3) << 21) + (uint32_t)((warp >> 2) * NT * 16);
+    pdl_trigger();
+  };
+  auto tmem_close = [&]() {
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+    asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory");
+    __syncthreads();
+    asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory");
+    if (warp == 0) asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(*sTmem), "r"(M::TCOLS));
+  };
 
   int row_tile, expert = 0;
   // raw column `col` of the row tile: pieces are dealt to consecutive threads along a row; rows past n re-read row n - 1,
@@ -164,6 +205,8 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
   // one tile: sTok / sDst hold `ntok` slots (a multiple of 8)
   auto run_tile = [&](int ntok, bool raw_issued) {
     const int ntiles = ntok >> 3;
+    const int every = p.nsb < 16 ? 1 : p.nsb < 64 ? 3 : 7;   // sums are closed after the sub-blocks whose index has these bits set
+    bool opened = false;                       // the tensor memory holds sums of this tile
     f2_t acc[2][NT][2];
 #pragma unroll
     for (int a = 0; a < 2; ++a)
@@ -265,11 +308,11 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
                     const float2 dv = f2_unpack(d), zv = f2_unpack(z);
                     const float2 pd = __half22float2(__floats2half2_rn(was[mt][hf] * dv.x, was[mt][hf] * dv.y));
                     const float2 pz = __half22float2(__floats2half2_rn(wbs[mt][hf] * zv.x, wbs[mt][hf] * zv.y));
-                    acc[mt][i][hf] = f2_fma(I, f2_pack(pd.x, pd.y), acc[mt][i][hf]);
-                    acc[mt][i][hf] = f2_add(acc[mt][i][hf], f2_pack(-pz.x, -pz.y));
+                    acc[mt][i][hf] = f2_add(acc[mt][i][hf], f2_fma(I, f2_pack(pd.x, pd.y), f2_pack(-pz.x, -pz.y)));
+                  } else if constexpr (F::HAS_MIN) {
+                    acc[mt][i][hf] = f2_add(acc[mt][i][hf], f2_fma(wa[mt][hf][0], f2_mul(I, d), f2_mul(wb[mt][hf][0], z)));
                   } else {
                     acc[mt][i][hf] = f2_fma(wa[mt][hf][0], f2_mul(I, d), acc[mt][i][hf]);
-                    if constexpr (F::HAS_MIN) acc[mt][i][hf] = f2_fma(wb[mt][hf][0], z, acc[mt][i][hf]);
                   }
                 }
               }
@@ -289,30 +332,61 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
 #pragma unroll
                 for (int hf = 0; hf < 2; ++hf) {
                   const f2_t I0 = f2_add(f2_bits(D0[2 * hf], D0[2 * hf + 1]), nmagic), I1 = f2_add(f2_bits(D1[2 * hf], D1[2 * hf + 1]), nmagic);
-                  acc[mt][i][hf] = f2_fma(d, f2_fma(wa[mt][hf][NG - 1], I1, f2_mul(wa[mt][hf][0], I0)), acc[mt][i][hf]);
-                  if constexpr (F::HAS_MIN) acc[mt][i][hf] = f2_fma(wb[mt][hf][NG - 1], z1, f2_fma(wb[mt][hf][0], z0, acc[mt][i][hf]));
+                  const f2_t dot = f2_fma(wa[mt][hf][NG - 1], I1, f2_mul(wa[mt][hf][0], I0));
+                  if constexpr (F::HAS_MIN) acc[mt][i][hf] = f2_add(acc[mt][i][hf], f2_fma(d, dot, f2_fma(wb[mt][hf][NG - 1], z1, f2_mul(wb[mt][hf][0], z0))));
+                  else acc[mt][i][hf] = f2_fma(d, dot, acc[mt][i][hf]);
                 }
               }
             }
           }
+        }
+        if (((4 * h + sub) & every) == every || (sub == 3 && h + 1 == nhalf)) {
+          // close these sub-blocks' sums: into {sum, correction} pairs in tensor memory, by Dekker's fast two-sum
+          if (opened) asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int i = 0; i < NT; ++i) {
+            if (i * WN + wn < ntiles) {
+              uint32_t v[16];
+              if (opened) {
+                mq_tmem_ld16(tacc + i * 16, v);
+              } else {
+#pragma unroll
+                for (int j = 0; j < 16; ++j) v[j] = 0u;
+              }
+#pragma unroll
+              for (int j = 0; j < 4; ++j) {
+                f2_t& c = acc[j >> 1][i][j & 1];
+                const f2_t sum = f2_bits((int)v[2 * j], (int)v[2 * j + 1]), minus1 = f2_pack(-1.0f, -1.0f);
+                const f2_t t = f2_add(sum, c), err = f2_fma(f2_fma(sum, minus1, t), minus1, c);   // c - (t - sum)
+                const f2_t corr = f2_add(f2_bits((int)v[8 + 2 * j], (int)v[9 + 2 * j]), err);
+                const float2 tv = f2_unpack(t), cv = f2_unpack(corr);
+                v[2 * j] = __float_as_uint(tv.x); v[2 * j + 1] = __float_as_uint(tv.y);
+                v[8 + 2 * j] = __float_as_uint(cv.x); v[9 + 2 * j] = __float_as_uint(cv.y);
+                c = 0ull;
+              }
+              mq_tmem_st16(tacc + i * 16, v);
+            }
+          }
+          opened = true;
         }
       }
     }
     // epilogue: transpose through shared memory (the buffers are free), lanes = consecutive rows of one token
     __syncthreads();
     float* sT = reinterpret_cast<float*>(mq_smem);     // [ROWS][65]: lanes = consecutive rows read without conflicts
+    asm volatile("tcgen05.wait::st.sync.aligned;" ::: "memory");
 #pragma unroll
     for (int i = 0; i < NT; ++i) {
       const int nt = i * WN + wn;
       if (nt < ntiles) {
+        uint32_t v[16];
+        mq_tmem_ld16(tacc + i * 16, v);
 #pragma unroll
-        for (int mt = 0; mt < 2; ++mt)
-#pragma unroll
-          for (int hf = 0; hf < 2; ++hf) {
-            const float2 v = f2_unpack(acc[mt][i][hf]);
-            float* at = sT + (wrow + mt * 16 + hf * 8 + g) * 65 + nt * 8 + 2 * t4;
-            at[0] = v.x; at[1] = v.y;
-          }
+        for (int j = 0; j < 8; ++j) {       // j: 16-row half, 8-row half, token of the pair
+          const float sum = __uint_as_float(v[j]);
+          // an infinite or NaN sum stays what it is
+          sT[(wrow + (j >> 2) * 16 + ((j >> 1) & 1) * 8 + g) * 65 + nt * 8 + 2 * t4 + (j & 1)] = isfinite(sum) ? sum + __uint_as_float(v[8 + j]) : sum;
+        }
       }
     }
     __syncthreads();
@@ -331,8 +405,8 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
       const int tok = t0 + tid < p.tokens ? t0 + tid : -1;
       sTok[tid] = tok; sDst[tid] = tok;
     }
-    __syncthreads();
     pdl_wait();
+    tmem_open();
     run_tile(ntok, true);
   } else {
     row_tile = blockIdx.x % p.row_tiles;
@@ -342,6 +416,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
     const int64_t npost = p.num_post_padded[0];
     int nblk = (int)((p.nslots + KQ_MOE_BLOCK - 1) / KQ_MOE_BLOCK);
     if (npost < 0) return;
+    tmem_open();
     if (npost / KQ_MOE_BLOCK + 1 < nblk) nblk = (int)(npost / KQ_MOE_BLOCK) + 1;   // blocks whose first slot is <= npost (moe.cuh:37)
     int run_start = 0, items = 0;            // of the block before the current one / items seen so far (the same in all warps)
     for (int base = 0; base < nblk; base += 32) {
@@ -376,6 +451,7 @@ __global__ void __launch_bounds__(MQ_THREADS, 2) mmq_kernel(const MmqParams p) {
       }
     }
   }
+  tmem_close();
 }
 
 template <int QT, bool MMQ, bool MOE, int ROWS>

@@ -67,3 +67,39 @@ def test_expert_runs(qt, e, n, tokens, top_k, one):
     s, ex, tot = (torch.from_numpy(a).to(dev()) for a in align(ids, 8, e))
     y = capi.moe_a8(wt, xt, s, ex, tot, top_k, qt, out_dtype=torch.float32)
     assert rel_l2(to_np(y), expected(w, qt, x, ids, "mmq")) < TIGHT
+
+
+def one_run(tokens):
+    """Sorted blocks of one expert's run: tokens 0 .. tokens - 1."""
+    s = np.full((tokens + 7) // 8 * 8, tokens, np.int32)
+    s[:tokens] = np.arange(tokens)
+    return [torch.from_numpy(a).to(dev()) for a in (s, np.zeros(s.size // 8, np.int32), np.array([s.size], np.int32))]
+
+
+@pytest.mark.parametrize("qt", O.ALL_QTYPES)
+@pytest.mark.parametrize("k", [256, 512, 5632])
+def test_fp32_error_is_not_above_the_kernels_it_stands_for(qt, k):
+    """Against the exact value, in fp32: the GEMV passes (formats without a tcgen05 GEMM) and the one-warp-per-row block op add a
+    row in 32 lanes and a tree.  3840 outputs: the two errors are known to about 1.1 %, so 5 % is three deviations of their ratio."""
+    n, m = 96, 40
+    w, wt = wire(qt, n, k, seed=qt + k)
+    x, xt = act(m, k, seed=k, dt="bf16")
+
+    def linear(new):
+        capi.set_option("mmq_min_m", 9 if new else 1 << 30)
+        try:
+            return capi.mul_mat(wt, xt, qt, mmq=qt not in O.NO_MMQ, out_dtype=torch.float32)
+        finally:
+            capi.set_option("mmq_min_m", 0)
+
+    def sorted_op(new):
+        capi.set_option("moe_smem", int(new))
+        try:
+            return capi.moe_a8(wt.view(1, n, -1), xt, *one_run(m), 1, qt, out_dtype=torch.float32)
+        finally:
+            capi.set_option("moe_smem", 1)
+
+    ref = O.mul_mat(w, qt, x, "mmvq" if qt in O.NO_MMQ else "mmq")
+    for call in ([linear] if qt in O.MORE_QTYPES else []) + ([sorted_op] if qt not in O.NO_MMQ else []):
+        old, new = rel_l2(to_np(call(False)), ref), rel_l2(to_np(call(True)), ref)
+        assert new <= 1.05 * old, (call.__name__, old, new)
