@@ -331,7 +331,9 @@ __device__ __forceinline__ uint32_t ld_u16x2(const uint8_t* p) {
 // N consecutive words from a 2-byte aligned address.  STAGED (shared memory holding the bytes at their address modulo 4, in a
 // window whose end is rounded up to a word at least): N + 1 aligned loads and a funnel shift per word instead of 2 N 16-bit
 // loads; the last of them reads the word that holds the final two bytes, never one past it.  Q8_0 at one token, 7168x5120:
-// 13.1 -> 11.8 us; with four words only (Q4_0, 8192x5120: 10.3 -> 10.7 us) the 16-bit loads stay.
+// 13.1 -> 11.8 us.  Q8_0 and Q6_K read their codes so; elsewhere the 16-bit loads are faster (us, 16-bit loads / words: Q4_0 8192x5120,
+// 1 token, 10.3 / 10.7; 17408x5120, 1 and 3 tokens, Q3_K 34.2 / 36.9 and 67.5 / 73.7, Q5_1 20.4 / 21.2 and 40.7 / 42.8; Q5_0
+// 5120x17408 20.6 / 21.5 and 41.1 / 43.9).
 template <int N, bool STAGED>
 __device__ __forceinline__ void ld_words(const uint8_t* p, uint32_t (&w)[N]) {
   if constexpr (STAGED) {
@@ -511,12 +513,10 @@ __device__ __forceinline__ void decode_subblock(const uint8_t* __restrict__ row,
   } else if constexpr (QT == KQ_TYPE_Q5_0 || QT == KQ_TYPE_Q5_1) {   // {half d, [half m,] qh[4], qs[16]}: 5-bit codes
     constexpr int HDR = QT == KQ_TYPE_Q5_0 ? 2 : 4;
     const uint8_t* b = row + (size_t)sb * (QT == KQ_TYPE_Q5_0 ? 22 : 24);
-    uint32_t qw[5];                                      // qh, then the nibbles
-    ld_words<5, STAGED>(b + HDR, qw);
-    const uint32_t qh = qw[0];
+    const uint32_t qh = ld_u16x2(b + HDR);
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-      const uint32_t w = qw[1 + i];
+      const uint32_t w = ld_u16x2(b + HDR + 4 + 4 * i);
       o.v[i] = (w & 0x0F0F0F0Fu) | nibble_to_bit4((qh >> (4 * i)) & 15u);
       o.v[i + 4] = ((w >> 4) & 0x0F0F0F0Fu) | nibble_to_bit4((qh >> (16 + 4 * i)) & 15u);
     }
@@ -527,13 +527,10 @@ __device__ __forceinline__ void decode_subblock(const uint8_t* __restrict__ row,
   } else if constexpr (QT == KQ_TYPE_Q3_K) {             // {hmask[32], qs[64], scales[12], half d}: 3-bit codes - 4
     const uint8_t* b = row + (size_t)(sb >> 3) * 110;
     const int j = sb & 7, n = j >> 2, jj = j & 3;
-    uint32_t qs[8], hm[8];
-    ld_words<8, STAGED>(b + 32 + 32 * n, qs);
-    ld_words<8, STAGED>(b, hm);
 #pragma unroll
     for (int i = 0; i < 8; ++i) {
-      const uint32_t lo = (qs[i] >> (2 * jj)) & 0x03030303u;
-      const uint32_t hb = (hm[i] >> (4 * n + jj)) & 0x01010101u;
+      const uint32_t lo = (ld_u16x2(b + 32 + 32 * n + 4 * i) >> (2 * jj)) & 0x03030303u;
+      const uint32_t hb = (ld_u16x2(b + 4 * i) >> (4 * n + jj)) & 0x01010101u;
       o.v[i] = sub4_bytes(lo | (hb << 2));
     }
     const float d = ld_h(b + 108);
