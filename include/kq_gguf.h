@@ -367,7 +367,8 @@ int kq_debug_copy_window(uint64_t base, int64_t n, int64_t rowbytes, int64_t row
  *                 tokens) instead of splitting K into row segments
  *   "moe_smem"    1 (default) = the per-pair MoE op stages a pair's activations in shared memory and the expert-sorted
  *                 block op runs as an integer GEMM (same exact dots, fp32 sums in another order), 0 = one warp per row
- *                 reading the activations from global memory
+ *                 reading the activations from global memory, 2 = as 1, with the weight rows of the per-pair op staged in
+ *                 shared memory wherever they fit instead of where that is faster (bit-identical results)
  *   "mmq_min_m"   smallest m at which the formats without a tcgen05 GEMM (Q4_1, Q5_0, Q5_1, Q3_K, Q5_K, IQ4_NL, IQ4_XS) run
  *                 as an integer GEMM instead of GEMV passes (0, the default: by the number of rows; exact integer dots either way)
  *   "gemm_wide"   tile of the GEMM: 0 = 256 rows x 128 tokens, 2 = 128 rows x 256 tokens, 1 (default) = the latter

@@ -608,7 +608,7 @@ int kq_set_option(const char* name, int value) {
   if (name && !strcmp(name, "gemm_wide")) { options().gemm_wide = value; return KQ_OK; }
   if (name && !strcmp(name, "gemm_small_m")) { options().gemm_small_m = value != 0; return KQ_OK; }
   if (name && !strcmp(name, "tile_two_stage")) { options().tile_two_stage = value != 0; return KQ_OK; }
-  if (name && !strcmp(name, "moe_smem")) { options().moe_smem = value != 0; return KQ_OK; }
+  if (name && !strcmp(name, "moe_smem")) { options().moe_smem = value == 2 ? 2 : value != 0; return KQ_OK; }
   if (name && !strcmp(name, "row_stage_kb")) { options().row_stage_kb = value < 4 ? 4 : (value > 96 ? 96 : value); return KQ_OK; }
   if (name && !strcmp(name, "mmq_min_m")) { options().mmq_min_m = value; return KQ_OK; }
   if (name && !strcmp(name, "umma")) { options().umma = value != 0; return KQ_OK; }

@@ -56,7 +56,8 @@ struct Options {
                        // or the format's wire bytes are staged through shared memory (where it is faster at every m)
   int row_stage_kb;    // Q4_K row-pair GEMV (1-2 tokens): target size of one ring stage (whole rows) in KB
   int tile_two_stage;  // 1: the shared-stage GEMV may run on two whole-row stages of >= 32 KB instead of splitting K
-  int moe_smem;        // 1: the MoE ops share activations through shared memory (block op: integer GEMM; 0: the one-warp-per-row kernel)
+  int moe_smem;        // 1: the MoE ops share activations through shared memory (block op: integer GEMM; 0: the one-warp-per-row kernel);
+                       // 2: as 1, and the per-pair op stages weight rows wherever they fit
   int gemm_small_m;    // 1: calls of 17..gemm_min_m-1 tokens also go to the tcgen05 GEMM where it beats the 16-token
                        // GEMV passes (staged formats, enough 128-row tiles to fill the GPU)
   int mmq_min_m;       // smallest token count at which the formats without a tcgen05 GEMM go to the integer GEMM

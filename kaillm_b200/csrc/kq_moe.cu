@@ -36,7 +36,7 @@ struct MoeParams {
   const int32_t* num_post_padded;    // block mode only
   int zero_bad;                      // vec: 1 = the output rows of pairs without a valid expert are written as zeros
   int64_t wbytes;                    // size of the whole weight tensor
-  int stages, stage_bytes;           // staged vec kernel: ring of row pairs per warp
+  int rows, stage_bytes;             // staged vec kernel: rows per CTA (a multiple of 16), bytes of one stage of a warp's ring
   int64_t nslots;                    // tokens * top_k (vec) / entries of sorted_token_ids (block)
   void* y;
   int64_t stride_y;
@@ -249,10 +249,12 @@ __device__ __forceinline__ void decode_staged(const uint8_t* row, int sb, const 
 
 // Vec mode with the weight rows staged as well: each warp runs its own ring of row pairs, filled by 16-byte cp.async pieces
 // of the aligned window around the two rows, so that 2-byte aligned blocks cost coalesced requests and the loads run
-// `stages - 1` pairs ahead of the arithmetic.  Same arithmetic and order of additions as above (bit-identical).
+// MOE_STAGES - 1 pairs ahead of the arithmetic.  Same arithmetic and order of additions as above (bit-identical).
+// A CTA takes 128 rows where that gives four CTAs per SM, otherwise 64 (eight pairs of rows in a row per warp leave few
+// calls enough CTAs: Q2_K 512x2048, 24 pairs, 30.9 us with 128 rows and 16.5 unstaged).
 // Measured: 32 pairs over 32 experts, Q4_K 2816x2048 and Q8_0 2048x1408 (the rows' bytes are 3.2 and 3.1 MB a pair): the
-// feed-forward call of 8 tokens 84.5 -> 69.9 us; unstaged the two kernels took 36 and 35 us, bound by their 2-byte loads.
-constexpr int MOE_STAGED_ROWS = 128;      // rows per CTA: eight pairs per warp
+// feed-forward call of 8 tokens 84.5 -> 61.3 us; unstaged the two kernels took 36 and 35 us, bound by their 2-byte loads.
+constexpr int MOE_STAGES = 3;             // row pairs in a warp's ring: one being multiplied, two on their way
 template <int QT, typename OutT>
 __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) {
   using F = Fmt<QT>;
@@ -262,7 +264,7 @@ __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) 
   int8_t* sQ = reinterpret_cast<int8_t*>(moe_smem);                          // [kpad]
   __half2* sDS = reinterpret_cast<__half2*>(moe_smem + p.kpad);              // [kpad / 32]
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
-  uint8_t* ring = moe_smem + p.kpad + nb8 * 4 + warp * p.stages * p.stage_bytes;
+  uint8_t* ring = moe_smem + p.kpad + nb8 * 4 + warp * MOE_STAGES * p.stage_bytes;
   const uint32_t ring_a = (uint32_t)__cvta_generic_to_shared(ring);
   pdl_trigger();
   if constexpr (QT == KQ_TYPE_IQ3_S) {
@@ -273,20 +275,20 @@ __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) 
   const int64_t z = blockIdx.y;                                              // the grid row is the (token, expert) pair
   const int expert = p.ids[z], tok = (int)(z / p.top_k);
   if (expert < 0 || expert >= p.experts) {
-    const int row = blockIdx.x * MOE_STAGED_ROWS + threadIdx.x;
-    if (p.zero_bad && threadIdx.x < MOE_STAGED_ROWS && row < p.n) y[(size_t)z * p.stride_y + row] = from_f32<OutT>(0.f);
+    const int row = blockIdx.x * p.rows + threadIdx.x;
+    if (p.zero_bad && threadIdx.x < p.rows && row < p.n) y[(size_t)z * p.stride_y + row] = from_f32<OutT>(0.f);
     return;
   }
   const uint8_t* We = p.W + (size_t)expert * p.expert_stride;
   const uint8_t* wend = p.W + p.wbytes;
-  const int row_end = min(p.n, (int)(blockIdx.x + 1) * MOE_STAGED_ROWS);
+  const int row_end = min(p.n, (int)(blockIdx.x + 1) * p.rows);
   auto issue = [&](int it) {              // rows row, row + 1 of this warp's it-th pair
-    const int row = blockIdx.x * MOE_STAGED_ROWS + 2 * (warp + 8 * it);
-    if (it < MOE_STAGED_ROWS / 16 && row < row_end) {
+    const int row = blockIdx.x * p.rows + 2 * (warp + 8 * it);
+    if (16 * it < p.rows && row < row_end) {
       const uint8_t* ga = We + (size_t)row * p.rowbytes;
       const uint8_t* a0 = reinterpret_cast<const uint8_t*>((uintptr_t)ga & ~(uintptr_t)15);
       const int bytes = (int)(ga - a0) + (row + 1 < row_end ? 2 : 1) * (int)p.rowbytes;
-      const uint32_t dst = ring_a + (it % p.stages) * p.stage_bytes;
+      const uint32_t dst = ring_a + (it % MOE_STAGES) * p.stage_bytes;
       for (int c = lane * 16; c < bytes; c += 512) {
         // of the tensor's last piece only the bytes that exist are read (the rest is zero-filled)
         const uint32_t have = a0 + c + 16 <= wend ? 16u : (uint32_t)(wend - (a0 + c));
@@ -295,7 +297,7 @@ __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) 
     }
     asm volatile("cp.async.commit_group;" ::: "memory");
   };
-  for (int i = 0; i < 2; ++i) issue(i);
+  for (int i = 0; i < MOE_STAGES - 1; ++i) issue(i);
   {
     const uint4* src = reinterpret_cast<const uint4*>(p.qs + (size_t)tok * p.kpad);
     for (int i = threadIdx.x; i < (p.kpad >> 4); i += blockDim.x) reinterpret_cast<uint4*>(sQ)[i] = __ldg(src + i);
@@ -303,13 +305,13 @@ __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) 
   }
   __syncthreads();
   constexpr int NG = 32 / F::GROUP;
-  for (int it = 0; it < MOE_STAGED_ROWS / 16; ++it) {
-    const int row = blockIdx.x * MOE_STAGED_ROWS + 2 * (warp + 8 * it);
+  for (int it = 0; 16 * it < p.rows; ++it) {
+    const int row = blockIdx.x * p.rows + 2 * (warp + 8 * it);
     if (row >= row_end) break;
-    asm volatile("cp.async.wait_group 1;" ::: "memory");
+    asm volatile("cp.async.wait_group %0;" ::"n"(MOE_STAGES - 2) : "memory");
     __syncwarp();                         // every lane's pieces of this pair have landed; everyone is past the pair before it
-    issue(it + 2);                        // into the buffer of the pair before it (three stages)
-    const uint8_t* w0 = ring + (it % p.stages) * p.stage_bytes + (((uint32_t)(uintptr_t)We + (uint32_t)row * (uint32_t)p.rowbytes) & 15u);
+    issue(it + MOE_STAGES - 1);           // into the buffer of the pair before it
+    const uint8_t* w0 = ring + (it % MOE_STAGES) * p.stage_bytes + (((uint32_t)(uintptr_t)We + (uint32_t)row * (uint32_t)p.rowbytes) & 15u);
     const int step = row + 1 < row_end ? (int)p.rowbytes : 0;               // a missing second row re-reads the first
     float acc[2] = {0.f, 0.f};
     for (int sb = lane; sb < p.nsb; sb += 32) {
@@ -358,6 +360,22 @@ __global__ void __launch_bounds__(256) moe_vec_staged_kernel(const MoeParams p) 
   }
 }
 
+// Staged rows (two CTAs share an SM) or the unstaged kernel?  Staging wins by the 2-byte loads it saves and the depth of its
+// loads, and loses by fewer warps per SM and a start-up of its own, so it pays where an expert's matrix is large and the block
+// awkward.  Staged / unstaged time of one call, geometric mean over eight shapes from 512x1024 to 5632x2048 x 1 to 256 pairs, weights from memory
+// and (in brackets) from L2: above the lines drawn here Q6_K 0.70 (0.72), Q3_K 0.71 (0.80), Q4_K 0.79 (0.86), Q5_K 0.80 (0.91), Q8_0 0.81
+// (0.82), Q5_1 0.81 (0.88), Q5_0 0.81 (0.94), Q2_K 0.87 (0.96), Q4_0 0.92 (0.94); below them up to 1.5 times slower.  Q4_1, IQ3_S, IQ4_NL
+// and IQ4_XS decode from aligned or few words: 1.1 to 1.4 times slower at 64 pairs and more.
+static bool moe_staged(int type, int64_t expert_bytes, int64_t pairs) {
+  if (options().moe_smem != 1) return options().moe_smem == 2;
+  switch (type) {
+    case KQ_TYPE_Q8_0: case KQ_TYPE_Q3_K: case KQ_TYPE_Q4_K: case KQ_TYPE_Q5_K: case KQ_TYPE_Q6_K: return expert_bytes >= 1000000;
+    case KQ_TYPE_Q4_0: case KQ_TYPE_Q5_1: case KQ_TYPE_Q2_K: return expert_bytes >= 1400000;
+    case KQ_TYPE_Q5_0: return expert_bytes >= 1400000 && pairs <= 32;
+    default: return false;
+  }
+}
+
 template <int QT, bool MMQ, typename OutT>
 int run_moe(const MoeParams& p, bool block, cudaStream_t st) {
   const unsigned gx = (unsigned)((p.n + 3) / 4);
@@ -371,16 +389,17 @@ int run_moe(const MoeParams& p, bool block, cudaStream_t st) {
     // three stages of a row pair and its aligned window (plus the word that a funnel shift reads past a block) per warp, where two
     // CTAs then share an SM
     MoeParams ps = p;
-    ps.stages = 3; ps.stage_bytes = (int)((2 * p.rowbytes + 14 + 4 + 15) / 16 * 16);
-    const size_t staged = smem + (size_t)8 * 3 * ps.stage_bytes;
-    if (p.nslots > 0 && staged <= 112 * 1024 && options().moe_smem && ((uintptr_t)p.W % 16) == 0) {
+    ps.stage_bytes = (int)((2 * p.rowbytes + 14 + 4 + 15) / 16 * 16);
+    const size_t staged = smem + (size_t)8 * MOE_STAGES * ps.stage_bytes;
+    if (p.nslots > 0 && staged <= 112 * 1024 && moe_staged(QT, p.expert_stride, p.nslots) && ((uintptr_t)p.W % 16) == 0) {
       auto kern = moe_vec_staged_kernel<QT, OutT>;
       static DeviceOnce staged_set;
       if (staged_set.first_time()) {
         KQ_CUDA_TRY(cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, 112 * 1024));
         staged_set.done();
       }
-      const unsigned gr = (unsigned)((p.n + MOE_STAGED_ROWS - 1) / MOE_STAGED_ROWS);
+      ps.rows = (p.n + 127) / 128 * p.nslots >= 4 * sm_count() ? 128 : 64;
+      const unsigned gr = (unsigned)((p.n + ps.rows - 1) / ps.rows);
       KQ_CUDA_TRY(launch_pdl(kern, dim3(gr, (unsigned)p.nslots), dim3(256), staged, st, options().pdl != 0, ps));
       options().launches += 1;
       KQ_CUDA_TRY(cudaGetLastError());
@@ -529,7 +548,7 @@ int launch_moe(const void* W, int type, int64_t experts, int64_t n, int64_t k, c
   int blk, bytes;
   if (!type_geometry(type, &blk, &bytes)) { set_error("unsupported GGML type %d", type); return KQ_EUNSUPPORTED; }
   MoeParams p;
-  p.W = (const uint8_t*)W; p.rowbytes = k / blk * bytes; p.expert_stride = p.rowbytes * n; p.wbytes = p.expert_stride * experts; p.stages = 0; p.stage_bytes = 0; p.n = (int)n; p.nsb = (int)(k / 32);
+  p.W = (const uint8_t*)W; p.rowbytes = k / blk * bytes; p.expert_stride = p.rowbytes * n; p.wbytes = p.expert_stride * experts; p.rows = 0; p.stage_bytes = 0; p.n = (int)n; p.nsb = (int)(k / 32);
   p.experts = (int)experts; p.ds = (const __half2*)ds; p.qs = (const int8_t*)qs; p.kpad = (int)kpad; p.tokens = (int)tokens;
   p.top_k = top_k; p.ids = ids; p.expert_ids = expert_ids; p.num_post_padded = num_post_padded; p.nslots = nslots;
   p.y = y; p.stride_y = stride_y; p.zero_bad = zero_bad;

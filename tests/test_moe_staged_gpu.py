@@ -29,3 +29,21 @@ def test_same_bits_as_the_unstaged_kernel(qt, n, k):
     finally:
         capi.set_option("moe_smem", 1)
     assert torch.equal(got, want) and not bool(got[3].any())
+
+
+@pytest.mark.parametrize("qt", O.ALL_QTYPES)
+@pytest.mark.parametrize("n,k,tokens", [(1, 256, 2), (63, 512, 3), (65, 1024, 3), (129, 2304, 5), (200, 256, 310)])
+def test_forced_staging_has_the_same_bits(qt, n, k, tokens):
+    """Edges of the 64-row tiles (128-row ones from 592 tiles on: the last shape), whatever the dispatch would choose."""
+    e, top_k = 3, 1
+    _, w = experts_wire(qt, e, n, k, seed=qt + n)
+    _, x = act(tokens, k, seed=k, dt="bf16")
+    idt = torch.from_numpy(routing(tokens, top_k, e, seed=n).astype(np.int32)).to(dev())
+    out = []
+    for mode in (0, 1, 2):
+        capi.set_option("moe_smem", mode)
+        try:
+            out.append(capi.moe_a8_vec(w, x, idt, qt, out_dtype=torch.float32))
+        finally:
+            capi.set_option("moe_smem", 1)
+    assert torch.equal(out[0], out[1]) and torch.equal(out[0], out[2])
