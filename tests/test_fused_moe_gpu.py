@@ -60,3 +60,30 @@ def test_invalid_expert_ids():
             only = linear.fused_moe_gguf(x[2:3], w1, w2, tw[2:3, :1].contiguous(), ids[2:3, :1].contiguous(), 12, 8)
             assert torch.equal(got[2:3], only)
     assert ops.ggml_moe_get_block_size(12) == 8
+
+
+@pytest.mark.parametrize("total,e,kind", [(8192, 2, "one"), (33, 7, "bad"), (5000, 1000, "bad"), (1025, 33, "skewed")])
+def test_align_kernel_order_and_invalid_ids(total, e, kind):
+    """Against the definition: slots of an expert in slot order, runs padded to 8, invalid ids in no run and flagged."""
+    rng = np.random.default_rng(total)
+    ids = np.full(total, 1) if kind == "one" else rng.integers(0, e, size=total)
+    if kind == "skewed":
+        ids = np.minimum(ids, rng.integers(0, e, size=total))
+    if kind == "bad":
+        ids[::5] = rng.choice([-1, e, 2 ** 31 - 1, -2 ** 31], size=ids[::5].size)
+    nb = (total + e * 7 + 7) // 8
+    want_s, want_e = [], []
+    for ex in range(e):
+        z = np.nonzero(ids == ex)[0]
+        pad = -z.size % 8
+        want_s += list(z) + [total] * pad
+        want_e += [ex] * ((z.size + pad) // 8)
+    post_want = len(want_s)
+    want_s += [total] * (8 * nb - len(want_s))
+    want_e += [-1] * (nb - len(want_e))
+    it = torch.from_numpy(ids.astype(np.int32)).to(dev())
+    s, ex, post = (torch.empty(n, dtype=torch.int32, device=dev()) for n in (8 * nb, nb, 2))
+    P, L = capi.ctypes.c_void_p, capi.ctypes.c_int64
+    assert capi.lib.kq_moe_align(P(it.data_ptr()), L(total), L(e), P(s.data_ptr()), L(8 * nb), P(ex.data_ptr()), L(nb), P(post.data_ptr()),
+                                 P(torch.cuda.current_stream().cuda_stream)) == 0
+    assert s.tolist() == want_s and ex.tolist() == want_e and post.tolist() == [post_want, int(kind == "bad")]
