@@ -21,9 +21,10 @@ _FLOATS = (torch.float32, torch.float16, torch.bfloat16)
 
 
 def _plain(x: torch.Tensor) -> bool:
-    """An ordinary 2-D tensor nobody differentiates, traces or batches: only then may an op without derivative and tracing
-    rules stand in for a chain of torch ops."""
+    """An ordinary 2-D tensor nobody differentiates, traces, batches or casts: only then may an op without derivative, tracing and
+    autocast rules stand in for a chain of torch ops (under autocast `sum` gives float32 and `@` the autocast type)."""
     return (type(x) is torch.Tensor and x.is_cuda and x.dim() == 2 and not torch.compiler.is_compiling()
+            and not torch.is_autocast_enabled("cuda")
             and not (x.requires_grad and torch.is_grad_enabled()) and not torch._C._functorch.is_functorch_wrapped_tensor(x)
             and torch.autograd.forward_ad.unpack_dual(x).tangent is None)
 
