@@ -308,6 +308,7 @@ int kq_read_status_static(int* status) {
   const uint8_t* scratch = (const uint8_t*)static_scratch_ptr(&rc);
   if (!scratch) return rc;
   // the status word sits at a fixed offset of the layout, whatever sizes the array was last used with
+  KQ_CUDA_TRY(cudaDeviceSynchronize());   // the copy below does not wait for non-blocking streams
   KQ_CUDA_TRY(cudaMemcpy(status, scratch + q8_layout(1, 1, 32).off_status, sizeof(int), cudaMemcpyDeviceToHost));
   return KQ_OK;
 }
@@ -364,6 +365,7 @@ int kq_dequant_mul_mat(const void* W, int type, int64_t n, int64_t k, const void
 
 int kq_dequant_mul_mat_status(int* status, int clear) {
   t_err[0] = 0;
+  KQ_CUDA_TRY(cudaDeviceSynchronize());   // the copy does not wait for non-blocking streams
   return dense_mm_status(status, clear);
 }
 
@@ -389,6 +391,7 @@ int kq_read_status(int type, int64_t m, int64_t n, int64_t k, const void* scratc
   if (!type_geometry(type, &b, &sz) || m <= 0 || n <= 0 || k <= 0 || !scratch || !status) { set_error("kq_read_status: bad argument"); return KQ_EINVAL; }
   const Q8Layout L = q8_layout(m, n, k);
   if (scratch_bytes < L.total) { set_error("kq_read_status: scratch too small"); return KQ_ESCRATCH; }
+  KQ_CUDA_TRY(cudaDeviceSynchronize());   // the copy below does not wait for non-blocking streams
   KQ_CUDA_TRY(cudaMemcpy(status, (const uint8_t*)scratch + L.off_status, sizeof(int), cudaMemcpyDeviceToHost));
   return KQ_OK;
 }
@@ -562,6 +565,7 @@ int kq_wait_arrival(const void* buf, size_t bytes, int dtype, int* status, void*
 
 int kq_arrival_status(int* failed, int clear) {
   t_err[0] = 0;
+  KQ_CUDA_TRY(cudaDeviceSynchronize());   // as above
   return arrival_status(failed, clear);
 }
 
