@@ -141,10 +141,15 @@ static int mul_mat(const char* fn, bool mmq, const void* W, int type, int64_t n,
   }
   if (gemm) return launch_gemm_tc(W, type, n, k, P, m, y, y_dtype, stride_y, mmq, st);
   // Formats without a tensor-core GEMM: from mmq_min_m tokens on one integer GEMM instead of GEMV passes of 8 tokens.  A
-  // 64-token tile costs about the same however few tokens it holds, so small matrices, whose passes are cheap, change over
-  // later (Q5_K, GEMV passes / integer GEMM, us: 12288x4096 17 tokens 70 / 66; 6144x5120 32 tokens 74 / 83, 64 tokens
-  // 144 / 109; 1024x4096 64 tokens 44 / 87, 100 tokens 70 / 87, 333 tokens 230 / 98)
-  const int64_t mq_m = n >= 8192 ? 24 : n >= 4096 ? 48 : n >= 2048 ? 80 : 128;
+  // 64-token tile costs about the same however few tokens it holds, and its time grows with K where a tile of a small matrix
+  // has an SM to itself; so small matrices, whose passes are cheap, change over later, and later still where K is long (Q5_K,
+  // GEMV passes / integer GEMM, us: K = 1024: 8192 rows 24 tokens 29 / 21, 2048 rows 80 tokens 46 / 28, 1024 rows 128 tokens 61 / 29;
+  // K = 5120: 12288 rows 24 tokens 99 / 90, 8192 rows 24 / 48 tokens 70 / 90 and 136 / 106, 6144 rows 48 tokens 110 / 106, 4096 rows
+  // 57 / 96 tokens 97 / 120 and 154 / 121, 3000 rows 89 tokens 134 / 121, 2048 rows 89 / 160 tokens 97 / 121 and 167 / 124, 1024 rows
+  // 137 / 256 tokens 107 / 123 and 194 / 130; Q4_1 at K = 2048 lies between)
+  const int64_t mq_short = n >= 8192 ? 24 : n >= 4096 ? 48 : n >= 2048 ? 80 : 128;
+  const int64_t mq_long = n >= 12288 ? 24 : n >= 8192 ? 40 : n >= 6144 ? 48 : n >= 4096 ? 72 : n >= 3000 ? 88 : n >= 2048 ? 112 : 176;
+  const int64_t mq_m = k < 2048 ? mq_short : mq_long;
   if (impl == 0 && m >= (options().mmq_min_m ? options().mmq_min_m : mq_m) && mmq_supported(W, type))
     return launch_mmq(W, type, n, k, P, m, y, y_dtype, stride_y, mmq, st);
   if (impl != 1 && gemv_mma_supported(W, type, n, k)) {

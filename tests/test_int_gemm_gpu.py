@@ -103,3 +103,15 @@ def test_fp32_error_is_not_above_the_kernels_it_stands_for(qt, k):
     for call in ([linear] if qt in O.MORE_QTYPES else []) + ([sorted_op] if qt not in O.NO_MMQ else []):
         old, new = rel_l2(to_np(call(False)), ref), rel_l2(to_np(call(True)), ref)
         assert new <= 1.05 * old, (call.__name__, old, new)
+
+
+@pytest.mark.parametrize("n,k,m,launches", [(2048, 5120, 89, 12), (2048, 1024, 89, 1), (2048, 5120, 112, 1), (8192, 5120, 33, 5), (8192, 5120, 40, 1)])
+def test_dispatch_looks_at_k(n, k, m, launches):
+    """Long rows of few-row matrices keep the GEMV passes (8 tokens each, then 4, 2, 1) longer: launches beside the quantizer's."""
+    qt = 13
+    _, wt = wire(qt, n, k, seed=1)
+    _, xt = act(m, k, seed=2, dt="bf16")
+    capi.mul_mat(wt, xt, qt, mmq=True)
+    before = capi.get_option("launch_count")
+    capi.mul_mat(wt, xt, qt, mmq=True)
+    assert capi.get_option("launch_count") - before == launches + 1
