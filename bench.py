@@ -624,7 +624,7 @@ def run_single(args, torch, dev, local):
                         us = tm.time(r, 5) * 1e3 / nm
                         gbs = algorithmic_bytes(qt, n, k, m) / us / 1e3
                         safe = (8 if n > 5120 else 16) if qt == IQ3_S else (2 if n > 5120 else 6)
-                        branch = "ggml_mul_mat_vec_a8" if m <= safe else ("ggml_mul_mat_a8" if qt != IQ3_S else "ggml_dequantize + torch matmul")
+                        branch = "ggml_mul_mat_vec_a8" if m <= safe else ("ggml_mul_mat_a8" if qt != IQ3_S else "ggml_dequant_mul_mat (one kernel where it covers the call)")
                         low.append({"type": NAMES[qt], "n": n, "k": k, "m": m, "branch": branch, "us_per_call": round(us, 2),
                                     "gbs": round(gbs, 1), "frac_of_measured_hbm": round(gbs / pk["hbm"], 3)})
                     del ws_

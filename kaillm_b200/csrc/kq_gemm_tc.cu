@@ -23,8 +23,8 @@
 //   warp 17   one lane issues the MMAs: per K step 8 x tcgen05.mma.kind::f16 (128 x 128 x 16) per row tile, A from TMEM,
 //             B through a shared-memory descriptor; tcgen05.commit signals "buffers free" and, at the end,
 //             "accumulators complete".
-//   TMEM: 256 accumulator columns (2 x 128) + an A ring of 2 slots x 128 columns; shared memory: a B ring of 5 steps x
-//   32 KB.  Every mbarrier wait is bounded; on give-up a status word is set, TMEM is released and the CTA returns.
+//   TMEM: at most 256 accumulator columns + 256 columns of A ring; shared memory: a B ring and a ring of weight columns (Tile and
+//   Rings below).  Every mbarrier wait is bounded; on give-up a status word is set, TMEM is released and the CTA returns.
 #include <type_traits>
 
 #include "kq_common.cuh"
@@ -82,7 +82,7 @@ struct GemmParams {
   int stage6;         // Q6_K: rows and W are 8-byte aligned, the block columns go through shared memory
   const __half* ctab;  // Q4_0: dense table [n][ctab_stride] of -8 * d per 32-block (null: read the scales from W)
   int64_t ctab_stride;
-  int stagew;         // Q8_0, Q4_0, Q2_K in the 128 x 256 tile: W is 16-byte aligned and k a multiple of 256, the columns go through shared memory
+  int stagew;         // window formats (Win below) in the wide tiles: W is 16-byte aligned and k a multiple of 256, the columns go through shared memory
 };
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }

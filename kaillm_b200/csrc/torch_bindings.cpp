@@ -261,7 +261,8 @@ at::Tensor fused_moe_swiglu(const at::Tensor& X, const at::Tensor& W1, const at:
     sorted = at::empty({nb * bs}, iopt); eids = at::empty({nb}, iopt); post = at::empty({2}, iopt);
     TORCH_CHECK(kq_moe_align(ids.data_ptr<int32_t>(), pairs, e, sorted.data_ptr<int32_t>(), nb * bs, eids.data_ptr<int32_t>(), nb,
                              post.data_ptr<int32_t>(), stream) == KQ_OK, fn, ": ", kq_last_error());
-    // an expert id outside [0, E) is an error in this branch: the flag travels to the host while the kernels below run
+    // an expert id outside [0, E) is an error in this branch: the flag travels to the host while the kernels below run, and the host
+    // waits for it (so for all earlier work of the stream) at the end of the call; not capturable, as the chain of ops is not either
     flag = at::empty({2}, at::TensorOptions().dtype(at::kInt).pinned_memory(true));
     flag.copy_(post, /*non_blocking=*/true);
     copied.record(at::cuda::getCurrentCUDAStream(X.get_device()));
