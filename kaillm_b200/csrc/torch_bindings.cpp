@@ -142,7 +142,10 @@ at::Tensor ggml_dequant_mul_mat(const at::Tensor& W, const at::Tensor& X, int64_
       X.dim() == 2 && X.stride(1) == 1 && W.size(0) == row && X.size(1) % blk == 0 && W.size(1) == X.size(1) / blk * bytes) {
     const int64_t m = X.size(0), k = X.size(1);
     const int xdt = kq_dtype_of(X.scalar_type(), fn);
-    if (kq_dequant_mul_mat_preferred(row, m) && kq_dequant_mul_mat_supported(W.data_ptr(), (int)type, row, k, X.data_ptr(), xdt, m, X.stride(0))) {
+    // short rows leave a second wave of tiles little to share its start-up with: 24576x1024 at 9 / 65 / 129 tokens, two steps / one kernel,
+    // us: IQ4_NL 27 / 29 / 31 against 31 / 33 / 35, IQ4_XS 29 / 30 / 32 against 32 / 33 / 35; 32000x1024 33 / 33 / 35 against 31 / 31 / 35
+    const bool short_rows = type != 21 && k < 2048 && row > 148 * 128 && row < 30000;   // IQ3_S: 31 against 29
+    if (!short_rows && kq_dequant_mul_mat_preferred(row, m) && kq_dequant_mul_mat_supported(W.data_ptr(), (int)type, row, k, X.data_ptr(), xdt, m, X.stride(0))) {
       const c10::cuda::CUDAGuard guard(X.device());
       at::Tensor Y = at::empty({m, row}, X.options());
       auto stream = at::cuda::getCurrentCUDAStream(X.get_device()).stream();
