@@ -76,6 +76,8 @@ class GGUFLinear:
     def _one_preparation(self, x: torch.Tensor) -> list[int] | None:
         """The op of every shard (0 mul_mat_vec, 1 mul_mat) where all of them multiply the same quantized activations: up to
         80 tokens (above, one GEMM operand is quantized per call anyway) and no shard on the dequantize-and-multiply branch."""
+        if x.shape[0] > 16 and any(t in IMATRIX_QUANT_TYPES for _, t in self.shards):   # cheap: the other checks took 2 to 4 us here
+            return None
         if not (_plain(x) and 0 < x.shape[0] <= 80 and x.stride(1) == 1 and x.dtype in _FLOATS):
             return None
         flavours = []
