@@ -143,7 +143,8 @@ static int mul_mat(const char* fn, bool mmq, const void* W, int type, int64_t n,
   // Formats without a tensor-core GEMM: from mmq_min_m tokens on one integer GEMM instead of GEMV passes of 8 tokens.  A
   // 64-token tile costs about the same however few tokens it holds, and its time grows with K where a tile of a small matrix
   // has an SM to itself; so small matrices, whose passes are cheap, change over later, and later still where K is long (Q5_K,
-  // GEMV passes / integer GEMM, us: K = 1024: 8192 rows 24 tokens 29 / 21, 2048 rows 80 tokens 46 / 28, 1024 rows 128 tokens 61 / 29;
+  // GEMV passes / integer GEMM, us, the latter as measured with one fp32 chain per output plus the 10 % that closing the sums
+  // costs: K = 1024: 8192 rows 24 tokens 29 / 21, 2048 rows 80 tokens 46 / 28, 1024 rows 128 tokens 61 / 29;
   // K = 5120: 12288 rows 24 tokens 99 / 90, 8192 rows 24 / 48 tokens 70 / 90 and 136 / 106, 6144 rows 48 tokens 110 / 106, 4096 rows
   // 57 / 96 tokens 97 / 120 and 154 / 121, 3000 rows 89 tokens 134 / 121, 2048 rows 89 / 160 tokens 97 / 121 and 167 / 124, 1024 rows
   // 137 / 256 tokens 107 / 123 and 194 / 130; Q4_1 at K = 2048 lies between)

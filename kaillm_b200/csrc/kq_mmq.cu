@@ -23,9 +23,9 @@
 //             is left: 0.57 / 0.69 / 0.72, and not above the replaced kernels' in any format from K = 256 on.  A
 //             sub-block's min term joins its dot before the chain.
 //
-// Measured (us, whole call, bf16 in and out, before -> now): Q5_K 6144x5120 at 64 / 100 / 333 tokens 144 / 229 / 755 -> 122 /
-// 123 / 219; Q3_K at 333 tokens 910 -> 229; the fused mixture-of-experts layer (32 experts, top 4, 2048/1408, Q4_K + Q8_0) at
-// 256 tokens 1057 -> 299.  What bounds it: latency of the half-column steps (load, decode, multiply behind barriers).
+// Measured (us, whole call, bf16 in and out, before -> now): Q5_K 6144x5120 at 333 tokens 755 -> 219
+// (197 with one fp32 chain per output); the fused mixture-of-experts layer (32 experts, top 4, 2048/1408, Q4_K + Q8_0) at
+// 256 tokens 1057 -> 300 (275).  What bounds it: latency of the half-column steps (load, decode, multiply behind barriers).
 //
 // Mixture of experts: a work item is a run of up to 8 consecutive 8-slot blocks of one expert; every CTA finds the items
 // from expert_ids itself and takes every gridDim-th of them.
